@@ -122,7 +122,7 @@ size_t Carve(cavs_treegru* e, void* base) {
   e->loss_scratch = w.Take<float>(LossHeadScratchBytes(c.hidden, c.classes) / sizeof(float));
   e->col_scratch = w.Take<float>(ColumnSumScratchBytes(3 * c.hidden) / sizeof(float));
   e->emb_scratch = w.Take<float>(MaxChunks(c) * 3 * H);
-  e->splitk_bytes = c.gemm_bf16 ? std::max(GemmBf16ScratchBytes(c.embed, 3 * c.hidden, 32), GemmBf16ScratchBytes(c.hidden, c.hidden, 32)) : 0;
+  e->splitk_bytes = c.gemm_bf16 ? std::max(GemmBf16ScratchBytes(c.embed, 3 * c.hidden, 32), GemmBf16ScratchBytes(c.hidden, c.hidden, 32)) : GemmF32ScratchBytes();
   e->splitk_scratch = w.Take<float>(e->splitk_bytes / sizeof(float));
   e->W_bf = w.Take<uint8_t>(c.gemm_bf16 ? E * 3 * H * 2 : 0);
   e->U_bf = w.Take<uint8_t>(c.gemm_bf16 ? 3 * H * H * 2 : 0);
@@ -152,6 +152,7 @@ int Gemm(cavs_treegru* e, void* c, long long ldc, int mode, const void* a, long 
   g.a = static_cast<const float*>(a); g.a_rs = a_t ? 1 : lda; g.a_cs = a_t ? lda : 1;
   g.b = static_cast<const float*>(b); g.b_rs = b_t ? 1 : ldb; g.b_cs = b_t ? ldb : 1;
   g.m = m; g.n = n; g.k = k;
+  g.scratch = e->splitk_scratch; g.scratch_bytes = e->splitk_bytes;
   return GemmF32(g, st);
 }
 

@@ -270,8 +270,7 @@ size_t IdxInts(const cavs_treelstm_config& c) {
 
 // Split-K scratch large enough for the three weight-gradient GEMMs at full capacity.
 size_t SplitKBytes(const cavs_treelstm_config& c) {
-  // fp32 mode: room for the k-split partials of a narrow level's products (up to 16 slabs of 64 rows x 4H)
-  if (!c.gemm_bf16) return static_cast<size_t>(16) * 64 * 4 * c.hidden * sizeof(float);
+  if (!c.gemm_bf16) return std::max(GemmF32ScratchBytes(), static_cast<size_t>(16) * 64 * 4 * c.hidden * sizeof(float));
   const int N = c.max_vertices, H = c.hidden, E = c.embed, K = c.n_slots;
   size_t b = GemmBf16ScratchBytes(E, 4 * H, 32);
   b = std::max(b, GemmBf16ScratchBytes(H, 3 * H, 32));

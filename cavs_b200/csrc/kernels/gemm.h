@@ -103,7 +103,7 @@ int GemmBf16SplitsForTile(int m, int n, int k, int tile_m);   // the same choice
 // is available: a third fewer operand bytes per flop out of L2.
 bool GemmBf16UsesTallTiles(int m, int n, int k, int a_major, int b_major, int out_mode);
 
-// fp32 GEMM on the CUDA cores with arbitrary element strides:
+// fp32 GEMM with arbitrary element strides, on the tensor cores (operands split into bf16 parts) or the CUDA cores:
 // C[i,j] (+)= sum_p A[i*a_rs + p*a_cs] * B[p*b_rs + j*b_cs].
 struct GemmF32Args {
   float* c = nullptr;
@@ -122,6 +122,11 @@ struct GemmF32Args {
   int k_per_split = 0;   // set by GemmF32 (0: no split)
 };
 int GemmF32(const GemmF32Args& args, cudaStream_t stream);
+// The tensor-core kernel alone: tiles of 128 x tile_n (128 or 64).  k is cut over *splits CTAs per tile (rewritten with
+// the number used); with more than one the partial products are left in args.scratch [splits, m, n].
+int GemmF32Split(const GemmF32Args& args, int tile_n, int* splits, cudaStream_t stream);
+// Scratch with which no product of a step is short of k splits: two partial tiles per SM.
+inline size_t GemmF32ScratchBytes() { return static_cast<size_t>(2) * 148 * 128 * 128 * sizeof(float); }
 
 }  // namespace cavs_b200
 #endif

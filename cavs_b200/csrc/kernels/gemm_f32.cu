@@ -1,9 +1,8 @@
-// fp32 GEMM on the CUDA cores (FFMA), used by the fp32 configurations whose results
-// must stay within 1e-5 relative of the reference's cublasSgemm calls
-// (cavs/backend/cublas_wrapper.cc:13-28): tcgen05 has no fp32-input MMA and TF32 keeps
-// only 10 mantissa bits.  These configurations are small and latency-bound: a 64x64x16
-// register-tiled kernel with element strides (any transpose without a copy) and a
-// software-pipelined k loop; the sum over k runs in ascending order within a thread.
+// fp32 GEMM, used by the fp32 configurations whose results must stay within 1e-5 relative of the reference's
+// cublasSgemm calls (cavs/backend/cublas_wrapper.cc:13-28): the choice between the tensor-core kernel on split operands
+// (gemm_f32_tc.cu) and, for products too small for it, the CUDA cores (FFMA) -- a 64x64x16 register-tiled kernel with
+// element strides (any transpose without a copy) and a software-pipelined k loop whose sum over k runs in ascending
+// order within a thread.
 #include <cstdint>
 
 #include "abi_common.h"
@@ -104,6 +103,7 @@ __global__ void __launch_bounds__(256) GemmF32Kernel(GemmF32Args g) {
 // C[i,j] (+)= sum over splits, in split order
 __global__ void __launch_bounds__(256) GemmF32Reduce(float* __restrict__ c, long long ldc, const float* __restrict__ part, int m, int n,
                                                      int splits, int accumulate) {
+  ChainAcquire();
   const long long total = static_cast<long long>(m) * n;
   for (long long i = static_cast<long long>(blockIdx.x) * 256 + threadIdx.x; i < total; i += static_cast<long long>(gridDim.x) * 256) {
     float acc = 0.0f;
@@ -111,6 +111,32 @@ __global__ void __launch_bounds__(256) GemmF32Reduce(float* __restrict__ c, long
     float* dst = c + (i / n) * ldc + (i % n);
     *dst = accumulate ? *dst + acc : acc;
   }
+}
+
+// k splits of the FFMA kernel: few tiles and a long k loop go to enough CTAs to fill the machine once (at least 64 k
+// per split).
+int PlainSplits(const GemmF32Args& g, long long tiles) {
+  if (g.scratch == nullptr || tiles >= SmCount() || g.k < 256) return 1;
+  int splits = static_cast<int>(std::min<long long>(std::min<long long>(16, g.k / 64), (2LL * SmCount()) / tiles));
+  while (splits > 1 && static_cast<size_t>(splits) * g.m * g.n * sizeof(float) > g.scratch_bytes) --splits;
+  return splits;
+}
+
+// Estimated microseconds, fitted to measurements of both kernels (B200, shapes from [20, 600] x 200 to [14474, 10000] x
+// 512, within 15 %).  Second pass over the partial products of a k split: launch + slabs in, result out.
+double ReduceCost(const GemmF32Args& g, int splits) {
+  return splits > 1 ? 2.0 + 4.0 * (splits + 1) * g.m * g.n / 3e6 : 0.0;
+}
+// FFMA: a 16-wide k step costs 0.92 us of latency, or 0.77 us of arithmetic for each CTA that shares the SM.
+double PlainCost(const GemmF32Args& g, long long tiles, int splits) {
+  const double steps = ((g.k + splits - 1) / splits + kTK - 1) / kTK;
+  return 3.5 + steps * std::max(0.92, 0.77 * ((tiles * splits + SmCount() - 1) / SmCount())) + ReduceCost(g, splits);
+}
+// Tensor cores: a 64-wide k block costs 2.2 us with 128 columns per tile, 1.95 us with 64.
+double SplitCost(const GemmF32Args& g, int tile_n, int splits) {
+  const long long items = static_cast<long long>((g.m + 127) / 128) * ((g.n + tile_n - 1) / tile_n) * splits;
+  const long long blocks = ((g.k + 63) / 64 + splits - 1) / splits, waves = (items + SmCount() - 1) / SmCount();
+  return 4.5 + waves * (0.8 + blocks * (tile_n == 128 ? 2.2 : 1.95)) + ReduceCost(g, splits);
 }
 
 }  // namespace
@@ -121,25 +147,35 @@ int GemmF32(const GemmF32Args& g_in, cudaStream_t stream) {
   if (g.m == 0 || g.n == 0) return CAVS_OK;
   CAVS_REQUIRE(g.a && g.b && g.c, CAVS_ERR_BAD_ARG, "gemm_f32: null pointer");
   dim3 grid((g.n + kTN - 1) / kTN, (g.m + kTM - 1) / kTM);
-  // Few tiles and a long k loop: split k over enough CTAs to fill the machine once (at least 64 k per split).
   const long long tiles = static_cast<long long>(grid.x) * grid.y;
-  int splits = 1;
-  if (g.scratch != nullptr && tiles < SmCount() && g.k >= 256) {
-    splits = static_cast<int>(std::min<long long>(std::min<long long>(16, g.k / 64), (2LL * SmCount()) / tiles));
-    while (splits > 1 && static_cast<size_t>(splits) * g.m * g.n * sizeof(float) > g.scratch_bytes) --splits;
-  }
+  int splits = PlainSplits(g, tiles);
+  // The cheaper kernel by the estimates above.  Both sides as measured (us, FFMA / tensor cores): [20, 600] x 200 14.7 /
+  // 13.4, [595, 450] x 150 12.8 / 12.6, [256, 1536] x 512 27 / 12.2 (4 k splits), [1500, 600] x 300 33 / 15.6, [400, 10000]
+  // x 200 84 / 36, [14474, 2048] x 512 1204 / 258; below one 64-wide k block the FFMA kernel is ahead.
+  int tc_tile = 0, tc_splits = 1;
+  double best = PlainCost(g, tiles, splits);
+  for (int tile : {128, 64})
+    for (int z = 1; z <= 32 && g.k > 0; z *= 2) {
+      if (z > 1 && (g.scratch == nullptr || z > (g.k + 63) / 64 || static_cast<size_t>(z) * g.m * g.n * sizeof(float) > g.scratch_bytes)) break;
+      const double cost = SplitCost(g, tile, z);
+      if (cost < best) { best = cost; tc_tile = tile; tc_splits = z; }
+    }
   g.k_per_split = 0;
-  if (splits > 1) {
-    g.k_per_split = ((g.k + splits - 1) / splits + kTK - 1) / kTK * kTK;
-    splits = (g.k + g.k_per_split - 1) / g.k_per_split;
-    grid.z = splits;
+  if (tc_tile > 0) {
+    splits = tc_splits;
+    if (int rc = GemmF32Split(g, tc_tile, &splits, stream)) return rc;
+  } else {
+    if (splits > 1) {
+      g.k_per_split = ((g.k + splits - 1) / splits + kTK - 1) / kTK * kTK;
+      splits = (g.k + g.k_per_split - 1) / g.k_per_split;
+      grid.z = splits;
+    }
+    GemmF32Kernel<<<grid, 256, 0, stream>>>(g);
+    CAVS_LAUNCH_CHECK("gemm_f32");
   }
-  GemmF32Kernel<<<grid, 256, 0, stream>>>(g);
-  CAVS_LAUNCH_CHECK("gemm_f32");
   if (splits > 1) {
-    GemmF32Reduce<<<GridForElems(static_cast<size_t>(g.m) * g.n, 256), 256, 0, stream>>>(g_in.c, g_in.ldc, g.scratch, g.m, g.n, splits,
-                                                                                          g_in.accumulate ? 1 : 0);
-    CAVS_LAUNCH_CHECK("gemm_f32 split reduce");
+    CAVS_CUDA(LaunchChained(GemmF32Reduce, dim3(GridForElems(static_cast<size_t>(g.m) * g.n, 256)), dim3(256), 0, stream, g_in.c,
+                            g_in.ldc, static_cast<const float*>(g.scratch), g.m, g.n, splits, g_in.accumulate ? 1 : 0));
   }
   return CAVS_OK;
 }
