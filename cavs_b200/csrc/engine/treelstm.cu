@@ -38,6 +38,7 @@
 #include "kernels/cell.h"
 #include "kernels/gemm.h"
 #include "kernels/launch.h"
+#include "kernels/narrow.h"
 
 using namespace cavs_b200;
 
@@ -58,6 +59,7 @@ struct cavs_treelstm {
   float* tail = nullptr;        // [0] loss sum, [1] status word (int)
   float *loss_scratch = nullptr, *col_scratch = nullptr, *emb_scratch = nullptr, *splitk_scratch = nullptr;
   size_t splitk_bytes = 0;
+  unsigned* barriers = nullptr;   // [4] grid-barrier words of the narrow levels' launches: forward 0..1, backward 2..3
   uint8_t *W_bf = nullptr, *U_bf = nullptr, *Wc_bf = nullptr;
   // wide loss head (classes > 8): logits / dz [N, Cp] fp32, bf16 copies of dz and of the pushed h rows
   float* logits = nullptr;
@@ -129,6 +131,7 @@ struct cavs_treelstm {
     // ascending order, and for each token segment its position in that list; n_xrows == 0: dense gradient block
     int32_t *xrows = nullptr, *seg_pos = nullptr;
     int n_xrows = 0;
+    int32_t *lev = nullptr;  // level offsets [n_levels + 1]
   };
   Batch slot[2];
   int active = -1, staged = -1;
@@ -263,7 +266,7 @@ size_t MaxLinkChunks(const cavs_treelstm_config& c) {
 }
 size_t IdxInts(const cavs_treelstm_config& c) {
   const size_t n = c.max_vertices;
-  return (2 * c.n_slots + 7) * n + 4 * (MaxChunks(c) + 1) + (MaxSegments(c) + 1) + 10 * MaxSegments(c) + 64 +
+  return (2 * c.n_slots + 8) * n + 2 + 4 * (MaxChunks(c) + 1) + (MaxSegments(c) + 1) + 10 * MaxSegments(c) + 64 +
          c.n_slots * n + 2 * (MaxLinkChunks(c) + 1) + 2 * (MaxSegments(c) + 1) +   // link lists (level 1 by token)
          static_cast<size_t>(std::max(c.vocab, 0)) + MaxSegments(c) + 2;            // exchange rows and their positions
 }
@@ -346,6 +349,7 @@ size_t Carve(cavs_treelstm* e, void* base) {
   e->emb_scratch = w.Take<float>(c.vocab == 0 ? 0 : MaxChunks(c) * 4 * H);
   e->splitk_bytes = SplitKBytes(c);
   e->splitk_scratch = w.Take<float>(e->splitk_bytes / sizeof(float));
+  e->barriers = w.Take<unsigned>(4);
   e->W_bf = w.Take<uint8_t>(c.gemm_bf16 ? static_cast<size_t>(E) * 4 * H * 2 : 0);
   e->U_bf = w.Take<uint8_t>(c.gemm_bf16 ? static_cast<size_t>(4) * H * H * 2 : 0);
   return w.used;
@@ -391,6 +395,38 @@ int Gemm(cavs_treelstm* e, void* c, long long ldc, int accumulate, const void* a
   g.scratch = e->splitk_scratch; g.scratch_bytes = e->splitk_bytes;
   PROF(e, kProfGemm, 2.0 * m * n * k, st, GemmF32(g, st));
   return CAVS_OK;
+}
+
+// Narrow levels of the fp32 configurations run as one persistent launch (kernels/narrow_f32.cu).  The level sizes of a
+// schedule do not increase, so they are a suffix of the levels: those whose fused multiply-adds the persistent kernel
+// (FFMA) finishes before the tensor-core products of the per-level path make up for its launches.  A per-level level
+// costs 25-35 us and direction whatever its size, FFMA about 45 us per 1e9 multiply-adds and tensor cores 25; the line
+// lies where the difference is 12 us.
+struct NarrowRange { int begin, end; NarrowPlan plan; };
+std::vector<NarrowRange> NarrowLevels(const cavs_treelstm* e, const cavs_treelstm::Batch& bt, bool backward) {
+  std::vector<NarrowRange> out;
+  if (e->bf16) return out;
+  const int H = e->cfg.hidden, K = e->cfg.n_slots;
+  auto rows = [&](int l) { return bt.level_off[l + 1] - bt.level_off[l]; };
+  int begin = 1;
+  while (begin < bt.n_levels && static_cast<double>(rows(begin)) * H * H * (3 + K) > 6e8) ++begin;
+  if (begin >= bt.n_levels) return out;
+  // Two launches when the upper levels are much narrower: few rows want few hidden units per CTA, so that all CTAs
+  // take part; many rows want many, so that a gathered row is used more often.
+  int split = begin;
+  while (split < bt.n_levels && rows(split) > 96) ++split;
+  const NarrowPlan wide = PlanNarrow(H, K, rows(begin), backward);
+  if (wide.w == 0) return out;
+  if (split > begin && bt.n_levels - split >= 4) {
+    const NarrowPlan low = PlanNarrow(H, K, rows(split), backward);
+    if (low.w != wide.w && low.w != 0) {
+      out.push_back({begin, split, wide});
+      out.push_back({split, bt.n_levels, low});
+      return out;
+    }
+  }
+  out.push_back({begin, bt.n_levels, wide});
+  return out;
 }
 
 }  // namespace
@@ -555,6 +591,7 @@ extern "C" int cavs_treelstm_load_batch(cavs_treelstm* e, const cavs_sched* s, c
   int32_t* h_tok = view(nt, &bt.tok);
   int32_t* h_label = view(nt, &bt.label);
   int32_t* h_order = view(nt, &bt.order);
+  std::memcpy(view(bt.level_off.size(), &bt.lev), bt.level_off.data(), bt.level_off.size() * sizeof(int32_t));
   int32_t* h_slot = view(nt, &bt.tok_slot);
   int32_t* h_child_st = e->leaf_tok ? view(static_cast<size_t>(K) * nt, &bt.child_st) : nullptr;
   int32_t* h_state_row = e->leaf_tok ? view(nt, &bt.state_row) : nullptr;
@@ -826,7 +863,10 @@ extern "C" int cavs_treelstm_forward(cavs_treelstm* e, void* stream) {
          LaunchEmbedFwd(e->X, e->bf16, Emb, bt.seg_tok, n_tok, E, e->cfg.vocab, st));
   }
   if ((rc = Gemm(e, e->A, 4 * H, pre, Xop, ldx, false, W, 4 * H, false, n_tok, 4 * H, E, false, st))) return rc;
-  for (int l = 0; l < bt.n_levels; ++l) {
+  const std::vector<NarrowRange> narrow = NarrowLevels(e, bt, false);
+  if (!narrow.empty()) CAVS_CUDA(cudaMemsetAsync(e->barriers, 0, 2 * sizeof(unsigned), st));
+  const int n_wide = narrow.empty() ? bt.n_levels : narrow.front().begin;   // levels launched one by one
+  for (int l = 0; l < n_wide; ++l) {
     const int off = bt.level_off[l], rows = bt.level_off[l + 1] - off;
     if (l == 0) {
       // leaf rows: read the token row's i,o,u blocks (3H) + its index, write h|c (2H); the gates are recomputed by
@@ -909,6 +949,18 @@ extern "C" int cavs_treelstm_forward(cavs_treelstm* e, void* stream) {
                        H, K, false, st));
   }
   ChainHint(false);
+  for (size_t i = 0; i < narrow.size(); ++i) {
+    NarrowForwardArgs na{};
+    na.state = e->state; na.gates = reinterpret_cast<float*>(e->gates);
+    na.S = reinterpret_cast<float*>(e->S); na.HK = reinterpret_cast<float*>(e->HK);
+    na.A = reinterpret_cast<const float*>(e->A); na.a_row = bt.tok_slot; na.bias = B;
+    na.U_iou = static_cast<const float*>(U_iou); na.U_f = static_cast<const float*>(U_f);
+    na.child = e->leaf_tok ? bt.child_st : bt.child; na.level_off = bt.lev;
+    na.barrier = e->barriers + i; na.status = e->Status();
+    na.n_total = nt; na.level_begin = narrow[i].begin; na.level_end = narrow[i].end; na.H = H;
+    const double rows = bt.level_off[narrow[i].end] - bt.level_off[narrow[i].begin];
+    PROF(e, kProfGemm, 2.0 * rows * H * H * (3 + K), st, LaunchNarrowForward(narrow[i].plan, na, K, st));
+  }
   (void)rc;
   // a forward-only caller may load the batch after next into this slot without ever running backward
   CAVS_CUDA(cudaEventRecord(e->slot_done[e->active], st));
@@ -991,7 +1043,23 @@ extern "C" int cavs_treelstm_backward(cavs_treelstm* e, void* stream) {
   const bool fuse_bias = tok_grad ? bt.shared_chunk >= 0 : CellBwdFusesBias(H);
   const size_t dB_rows = static_cast<size_t>(CellBwdMaxGrid());
   if (fuse_bias) CAVS_CUDA(cudaMemsetAsync(e->dB_tmp, 0, dB_rows * 4 * H * sizeof(float), st));
-  for (int l = bt.n_levels - 1; l >= (tok_grad ? 1 : 0); --l) {
+  const std::vector<NarrowRange> narrow = NarrowLevels(e, bt, true);
+  if (!narrow.empty()) CAVS_CUDA(cudaMemsetAsync(e->barriers + 2, 0, 2 * sizeof(unsigned), st));
+  for (size_t i = narrow.size(); i-- > 0;) {
+    NarrowBackwardArgs na{};
+    na.dA = reinterpret_cast<float*>(e->dA); na.ZF = reinterpret_cast<float*>(e->ZF); na.mailbox = e->mailbox;
+    na.dB_part = fuse_bias ? e->dB_tmp : nullptr;
+    na.dOut = e->FusedDh() ? nullptr : (e->Headless() ? e->dh_ext : e->dOut);
+    na.dz = e->FusedDh() ? e->dz8 : nullptr; na.Wc = e->params + e->OffWc(); na.C = C;
+    na.gates = reinterpret_cast<const float*>(e->gates); na.state = e->state;
+    na.U_iou = static_cast<const float*>(U_iou); na.U_f = static_cast<const float*>(U_f);
+    na.child = bt.child; na.child_state = e->leaf_tok ? bt.child_st : nullptr; na.parent = bt.parent; na.level_off = bt.lev;
+    na.barrier = e->barriers + 2 + i; na.status = e->Status();
+    na.n_total = nt; na.level_begin = narrow[i].begin; na.level_end = narrow[i].end; na.H = H;
+    const double rows = bt.level_off[narrow[i].end] - bt.level_off[narrow[i].begin];
+    PROF(e, kProfGemm, 2.0 * rows * H * H * (3 + K), st, LaunchNarrowBackward(narrow[i].plan, na, K, st));
+  }
+  for (int l = (narrow.empty() ? bt.n_levels : narrow.front().begin) - 1; l >= (tok_grad ? 1 : 0); --l) {
     const int off = bt.level_off[l], rows = bt.level_off[l + 1] - off;
     // read d(h) (H; or the dz row with the fused head), mailbox (2H), gates, own c (H) [+ child c (KH)];
     // write dA (4H) [+ ZF (KH), child dc (KH)]

@@ -176,6 +176,7 @@ int GemmF32(const GemmF32Args& g_in, cudaStream_t stream) {
   if (splits > 1) {
     CAVS_CUDA(LaunchChained(GemmF32Reduce, dim3(GridForElems(static_cast<size_t>(g.m) * g.n, 256)), dim3(256), 0, stream, g_in.c,
                             g_in.ldc, static_cast<const float*>(g.scratch), g.m, g.n, splits, g_in.accumulate ? 1 : 0));
+    CAVS_LAUNCH_CHECK("gemm_f32 split reduce");
   }
   return CAVS_OK;
 }

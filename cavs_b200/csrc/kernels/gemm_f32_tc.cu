@@ -435,6 +435,7 @@ int LaunchSplit(const SplitParams& p, cudaStream_t stream) {
   const long long work = static_cast<long long>((p.g.m + kBM - 1) / kBM) * ((p.g.n + kBN - 1) / kBN) * p.n_splits;
   const int grid = static_cast<int>(std::min<long long>(work, SmCount()));
   CAVS_CUDA(LaunchChained(GemmF32SplitKernel<kBN, kModeA, kModeB>, dim3(grid), dim3(kF32Threads), bytes, stream, p));
+  CAVS_LAUNCH_CHECK("gemm_f32 split");
   return CAVS_OK;
 }
 template <int kBN, int kModeA>
