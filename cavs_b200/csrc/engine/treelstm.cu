@@ -108,6 +108,7 @@ struct cavs_treelstm {
   // G3 [N,3H] (i|o|u, the head of `gates`) and GF [N,K,H] (forget gates, behind it); P and Q are never stored, and
   // the forward cell only forms c and h.  CAVS_GATE_EPILOGUE=0 keeps the separate pre-activation arrays.
   bool gate_epi = false;
+  bool narrow = true;          // narrow levels in one persistent launch (CAVS_NARROW_LEVELS=0: level by level)
   bool dual_gemm = true;       // small levels: both products of a level in one launch (CAVS_DUAL_GEMM=0: never)
   uint8_t* gates_f = nullptr;
   TcOperandMap map_G3, map_GF;
@@ -298,6 +299,8 @@ void InitModes(cavs_treelstm* e, const cavs_treelstm_config& cfg) {
   e->l1_always = v1 != nullptr && v1[0] == '1';
   const char* v3 = std::getenv("CAVS_DUAL_GEMM");
   e->dual_gemm = !(v3 != nullptr && v3[0] == '0');
+  const char* v4 = std::getenv("CAVS_NARROW_LEVELS");
+  e->narrow = !(v4 != nullptr && v4[0] == '0');
   const char* v2 = std::getenv("CAVS_GATE_EPILOGUE");
   e->gate_epi = e->bf16 && cfg.hidden % 64 == 0 && !(v2 != nullptr && v2[0] == '0');
 }
@@ -397,28 +400,37 @@ int Gemm(cavs_treelstm* e, void* c, long long ldc, int accumulate, const void* a
   return CAVS_OK;
 }
 
-// Narrow levels of the fp32 configurations run as one persistent launch (kernels/narrow_f32.cu).  The level sizes of a
-// schedule do not increase, so they are a suffix of the levels: those whose fused multiply-adds the persistent kernel
-// (FFMA) finishes before the tensor-core products of the per-level path make up for its launches.  A per-level level
-// costs 25-35 us and direction whatever its size, FFMA about 45 us per 1e9 multiply-adds and tensor cores 25; the line
-// lies where the difference is 12 us.
+// Narrow levels run as one persistent launch (kernels/narrow_f32.cu, narrow_bf16.cu).  The level sizes of a schedule do
+// not increase, so they are a suffix of the levels: from the first one that the persistent kernel is estimated to finish
+// sooner than the per-level launches.
+// fp32: a per-level level costs 25 us forward and 31 backward up to some hundred rows; the persistent one 4 and 9 us and
+// 1 us per 7e6 (forward) or 3.3e6 (backward) multiply-adds (H = 512, one child slot): the line lies below where they meet.
+// bf16: per level 16 us forward and 23 us backward at H = 512, 18 and 30 at 1024 (launch and fill floors).
 struct NarrowRange { int begin, end; NarrowPlan plan; };
 std::vector<NarrowRange> NarrowLevels(const cavs_treelstm* e, const cavs_treelstm::Batch& bt, bool backward) {
   std::vector<NarrowRange> out;
-  if (e->bf16) return out;
   const int H = e->cfg.hidden, K = e->cfg.n_slots;
   auto rows = [&](int l) { return bt.level_off[l + 1] - bt.level_off[l]; };
-  int begin = 1;
-  while (begin < bt.n_levels && static_cast<double>(rows(begin)) * H * H * (3 + K) > 6e8) ++begin;
+  int begin = bt.l1 ? 2 : 1;
+  if (!e->narrow) return out;
+  if (e->bf16) {
+    const double per_level = backward ? 16.0 + H / 75.0 : 13.0 + H / 200.0;
+    while (begin < bt.n_levels && rows(begin) > 0 && PlanNarrowBf16(H, K, rows(begin), backward).level_us > 0.8 * per_level) ++begin;
+    if (begin >= bt.n_levels) return out;
+    const NarrowPlan plan = PlanNarrowBf16(H, K, rows(begin), backward);
+    if (plan.w != 0) out.push_back({begin, bt.n_levels, plan});
+    return out;
+  }
+  while (begin < bt.n_levels && static_cast<double>(rows(begin)) * H * H * (3 + K) > (backward ? 6e7 : 1.2e8)) ++begin;
   if (begin >= bt.n_levels) return out;
   // Two launches when the upper levels are much narrower: few rows want few hidden units per CTA, so that all CTAs
   // take part; many rows want many, so that a gathered row is used more often.
   int split = begin;
   while (split < bt.n_levels && rows(split) > 96) ++split;
-  const NarrowPlan wide = PlanNarrow(H, K, rows(begin), backward);
+  const NarrowPlan wide = PlanNarrowF32(H, K, rows(begin), backward);
   if (wide.w == 0) return out;
   if (split > begin && bt.n_levels - split >= 4) {
-    const NarrowPlan low = PlanNarrow(H, K, rows(split), backward);
+    const NarrowPlan low = PlanNarrowF32(H, K, rows(split), backward);
     if (low.w != wide.w && low.w != 0) {
       out.push_back({begin, split, wide});
       out.push_back({split, bt.n_levels, low});
@@ -951,15 +963,15 @@ extern "C" int cavs_treelstm_forward(cavs_treelstm* e, void* stream) {
   ChainHint(false);
   for (size_t i = 0; i < narrow.size(); ++i) {
     NarrowForwardArgs na{};
-    na.state = e->state; na.gates = reinterpret_cast<float*>(e->gates);
-    na.S = reinterpret_cast<float*>(e->S); na.HK = reinterpret_cast<float*>(e->HK);
-    na.A = reinterpret_cast<const float*>(e->A); na.a_row = bt.tok_slot; na.bias = B;
-    na.U_iou = static_cast<const float*>(U_iou); na.U_f = static_cast<const float*>(U_f);
+    na.state = e->state; na.gates = e->gates; na.S = e->S; na.HK = e->HK;
+    na.gates_f = e->gates_f ? e->gates_f : e->gates + static_cast<size_t>(3) * H * e->elt;
+    na.pitch3 = (e->gates_f ? 3 : 3 + K) * H; na.pitch_f = (e->gates_f ? K : 3 + K) * H;
+    na.A = e->A; na.a_row = bt.tok_slot; na.bias = B; na.U_iou = U_iou; na.U_f = U_f;
     na.child = e->leaf_tok ? bt.child_st : bt.child; na.level_off = bt.lev;
     na.barrier = e->barriers + i; na.status = e->Status();
     na.n_total = nt; na.level_begin = narrow[i].begin; na.level_end = narrow[i].end; na.H = H;
     const double rows = bt.level_off[narrow[i].end] - bt.level_off[narrow[i].begin];
-    PROF(e, kProfGemm, 2.0 * rows * H * H * (3 + K), st, LaunchNarrowForward(narrow[i].plan, na, K, st));
+    PROF(e, kProfGemm, 2.0 * rows * H * H * (3 + K), st, e->bf16 ? LaunchNarrowForwardBf16(narrow[i].plan, na, K, st) : LaunchNarrowForwardF32(narrow[i].plan, na, K, st));
   }
   (void)rc;
   // a forward-only caller may load the batch after next into this slot without ever running backward
@@ -1047,17 +1059,18 @@ extern "C" int cavs_treelstm_backward(cavs_treelstm* e, void* stream) {
   if (!narrow.empty()) CAVS_CUDA(cudaMemsetAsync(e->barriers + 2, 0, 2 * sizeof(unsigned), st));
   for (size_t i = narrow.size(); i-- > 0;) {
     NarrowBackwardArgs na{};
-    na.dA = reinterpret_cast<float*>(e->dA); na.ZF = reinterpret_cast<float*>(e->ZF); na.mailbox = e->mailbox;
+    na.dA = e->dA; na.ZF = e->ZF; na.mailbox = e->mailbox;
     na.dB_part = fuse_bias ? e->dB_tmp : nullptr;
     na.dOut = e->FusedDh() ? nullptr : (e->Headless() ? e->dh_ext : e->dOut);
     na.dz = e->FusedDh() ? e->dz8 : nullptr; na.Wc = e->params + e->OffWc(); na.C = C;
-    na.gates = reinterpret_cast<const float*>(e->gates); na.state = e->state;
-    na.U_iou = static_cast<const float*>(U_iou); na.U_f = static_cast<const float*>(U_f);
+    na.gates = e->gates; na.state = e->state; na.U_iou = U_iou; na.U_f = U_f;
+    na.gates_f = e->gates_f ? e->gates_f : e->gates + static_cast<size_t>(3) * H * e->elt;
+    na.pitch3 = (e->gates_f ? 3 : 3 + K) * H; na.pitch_f = (e->gates_f ? K : 3 + K) * H;
     na.child = bt.child; na.child_state = e->leaf_tok ? bt.child_st : nullptr; na.parent = bt.parent; na.level_off = bt.lev;
     na.barrier = e->barriers + 2 + i; na.status = e->Status();
     na.n_total = nt; na.level_begin = narrow[i].begin; na.level_end = narrow[i].end; na.H = H;
     const double rows = bt.level_off[narrow[i].end] - bt.level_off[narrow[i].begin];
-    PROF(e, kProfGemm, 2.0 * rows * H * H * (3 + K), st, LaunchNarrowBackward(narrow[i].plan, na, K, st));
+    PROF(e, kProfGemm, 2.0 * rows * H * H * (3 + K), st, e->bf16 ? LaunchNarrowBackwardBf16(narrow[i].plan, na, K, st) : LaunchNarrowBackwardF32(narrow[i].plan, na, K, st));
   }
   for (int l = (narrow.empty() ? bt.n_levels : narrow.front().begin) - 1; l >= (tok_grad ? 1 : 0); --l) {
     const int off = bt.level_off[l], rows = bt.level_off[l + 1] - off;

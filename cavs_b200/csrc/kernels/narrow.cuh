@@ -1,0 +1,179 @@
+// What the persistent launches over narrow levels share in fp32 (narrow_f32.cu) and bf16 (narrow_bf16.cu): the grid
+// barrier, the gate gradients of the backward pass, the cooperative launch.
+#ifndef CAVS_B200_KERNELS_NARROW_CUH_
+#define CAVS_B200_KERNELS_NARROW_CUH_
+
+#include <cuda_bf16.h>
+#include <cuda_fp16.h>
+
+#include <cstdint>
+
+#include "abi_common.h"
+#include "kernels/cell.h"
+#include "kernels/launch.h"
+#include "kernels/narrow.h"
+
+namespace cavs_b200 {
+namespace narrow {
+
+constexpr int kThreads = 512, kWarps = kThreads / 32;
+constexpr size_t kMaxSmem = 226 * 1024;
+constexpr unsigned kBarrierPolls = 1u << 19;   // about half a second
+
+// The cell kernels' activations (kernels/cell.cu): libm-accurate for fp32, exp2-unit forms for bf16.
+template <bool kFast>
+__device__ __forceinline__ float Sigmoid(float x) { return kFast ? __fdividef(1.0f, 1.0f + __expf(-x)) : 1.0f / (1.0f + expf(-x)); }
+template <bool kFast>
+__device__ __forceinline__ float Tanh(float x) { return kFast ? 1.0f - __fdividef(2.0f, __expf(2.0f * x) + 1.0f) : tanhf(x); }
+
+__device__ __forceinline__ float LoadCg(const float* p) { return __ldcg(p); }
+__device__ __forceinline__ float LoadCg(const __half* p) { return __half2float(__ushort_as_half(__ldcg(reinterpret_cast<const unsigned short*>(p)))); }
+__device__ __forceinline__ void StoreAs(float* p, float x) { *p = x; }
+__device__ __forceinline__ void StoreAs(__nv_bfloat16* p, float x) { *p = __float2bfloat16_rn(x); }
+__device__ __forceinline__ void StoreAs(__half* p, float x) { *p = __float2half_rn(x); }
+
+// All CTAs of the grid (launched cooperatively) arrive; false, and *status raised, if that takes too long.
+__device__ __forceinline__ bool GridSync(unsigned* counter, unsigned target, int* status) {
+  __shared__ int s_ok;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    asm volatile("fence.acq_rel.gpu;" ::: "memory");
+    asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(counter) : "memory");
+    int ok = 0;
+    for (unsigned it = 0; it < kBarrierPolls; ++it) {
+      unsigned v;
+      asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(counter) : "memory");
+      if (v >= target) { ok = 1; break; }
+    }
+    asm volatile("fence.acq_rel.gpu;" ::: "memory");
+    if (!ok) atomicExch(status, 1);
+    s_ok = ok;
+  }
+  __syncthreads();
+  return s_ok != 0;
+}
+
+// First phase of a backward level, gate gradients: a thread owns one hidden column and every row_step-th row of each
+// level, so the column sums for the bias gradient stay in its registers.  Expressions and order are CellBwd's.
+// TG: type of the saved gates, TD: type of dA and ZF.
+constexpr int kColBlock = 64, kRowLanes = kThreads / kColBlock;
+template <int K, typename TG, typename TD>
+struct GateGradients {
+  static constexpr bool kFast = sizeof(TD) == 2;
+  int j, row0, row_step;
+  bool owner;
+  float sums[4], wc[kHeadDzPitch];
+  // of the next row, everything but its mailbox row
+  int ch[K];
+  bool has_parent;
+  float gi, go, gu, cown, d_out, gf[K], cch[K];
+
+  __device__ __forceinline__ explicit GateGradients(const NarrowBackwardArgs& a) {
+    const int col_blocks = (a.H + kColBlock - 1) / kColBlock, strips = max(1, static_cast<int>(gridDim.x) / col_blocks);
+    const int strip = blockIdx.x / col_blocks;
+    j = (blockIdx.x % col_blocks) * kColBlock + threadIdx.x % kColBlock;
+    row0 = strip * kRowLanes + static_cast<int>(threadIdx.x) / kColBlock;
+    row_step = strips * kRowLanes;
+    owner = j < a.H && strip < strips;
+#pragma unroll
+    for (int g = 0; g < 4; ++g) sums[g] = 0.0f;
+#pragma unroll
+    for (int c = 0; c < kHeadDzPitch; ++c) wc[c] = owner && a.dz != nullptr && c < a.C ? a.Wc[static_cast<size_t>(c) * a.H + j] : 0.0f;
+  }
+  __device__ __forceinline__ void Fetch(const NarrowBackwardArgs& a, size_t t) {
+    const int H = a.H;
+    has_parent = __ldg(a.parent + t) >= 0;
+    const TG* g = static_cast<const TG*>(a.gates) + t * a.pitch3 + j;
+    const TG* f = static_cast<const TG*>(a.gates_f) + t * a.pitch_f + j;
+    gi = LoadCg(g); go = LoadCg(g + H); gu = LoadCg(g + 2 * H);
+    cown = __ldcg(a.state + t * 2 * H + H + j);
+#pragma unroll
+    for (int c = 0; c < K; ++c) {
+      ch[c] = __ldg(a.child + static_cast<size_t>(c) * a.n_total + t);
+      const int chs = a.child_state ? __ldg(a.child_state + static_cast<size_t>(c) * a.n_total + t) : ch[c];
+      gf[c] = LoadCg(f + c * H);
+      cch[c] = ch[c] >= 0 ? __ldcg(a.state + static_cast<size_t>(chs) * 2 * H + H + j) : 0.0f;
+    }
+    d_out = 0.0f;
+    if (a.dz != nullptr) {
+#pragma unroll
+      for (int c = 0; c < kHeadDzPitch; ++c)
+        if (c < a.C) d_out = fmaf(__ldg(a.dz + t * kHeadDzPitch + c), wc[c], d_out);
+    } else {
+      d_out = __ldg(a.dOut + t * H + j);
+    }
+  }
+  // Requests the first row of a level whose mailbox rows are not complete yet.
+  __device__ __forceinline__ void Request(const NarrowBackwardArgs& a, int off, int end) {
+    if (owner && off + row0 < end) Fetch(a, off + row0);
+  }
+  __device__ __forceinline__ void Level(const NarrowBackwardArgs& a, int off, int end) {
+    if (!owner) return;
+    const int H = a.H;
+    for (int t_ = off + row0; t_ < end; t_ += row_step) {
+      const size_t t = t_;
+      const float mh = has_parent ? __ldcg(a.mailbox + t * 2 * H + j) : 0.0f, mc = has_parent ? __ldcg(a.mailbox + t * 2 * H + H + j) : 0.0f;
+      const GateGradients x = *this;
+      if (t_ + row_step < end) Fetch(a, t_ + row_step);   // beside this row's mailbox
+      const float dh = x.d_out + mh, th = Tanh<kFast>(x.cown), d_o = dh * th;
+      const float dc = mc + (dh * x.go) * (1.0f - th * th);
+      const float zi = (dc * x.gu) * x.gi * (1.0f - x.gi), zo = d_o * x.go * (1.0f - x.go), zu = (dc * x.gi) * (1.0f - x.gu * x.gu);
+      float zfs = 0.0f;
+      TD* zf = static_cast<TD*>(a.ZF) + t * K * H + j;
+#pragma unroll
+      for (int c = 0; c < K; ++c) {
+        float z = 0.0f;
+        if (x.ch[c] >= 0) {
+          z = (dc * x.cch[c]) * x.gf[c] * (1.0f - x.gf[c]);
+          zfs += z;
+          a.mailbox[static_cast<size_t>(x.ch[c]) * 2 * H + H + j] = dc * x.gf[c];
+        }
+        StoreAs(zf + c * H, z);
+      }
+      TD* d = static_cast<TD*>(a.dA) + t * 4 * H + j;
+      StoreAs(d, zi); StoreAs(d + H, zo); StoreAs(d + 2 * H, zu); StoreAs(d + 3 * H, zfs);
+      sums[0] += zi; sums[1] += zo; sums[2] += zu; sums[3] += zfs;
+    }
+  }
+  // Column sums of this CTA's rows, row lanes folded in order, into its row of dB_part; scratch: 4 x kThreads floats.
+  __device__ __forceinline__ void FoldSums(const NarrowBackwardArgs& a, float* scratch) {
+    if (a.dB_part == nullptr) return;
+    __syncthreads();
+#pragma unroll
+    for (int g = 0; g < 4; ++g) scratch[g * kThreads + threadIdx.x] = sums[g];
+    __syncthreads();
+    if (!owner || threadIdx.x >= kColBlock) return;
+#pragma unroll
+    for (int g = 0; g < 4; ++g) {
+      float acc = 0.0f;
+      for (int r = 0; r < kRowLanes; ++r) acc += scratch[g * kThreads + r * kColBlock + threadIdx.x];
+      a.dB_part[static_cast<size_t>(blockIdx.x) * 4 * a.H + g * a.H + j] += acc;
+    }
+  }
+};
+
+template <auto kKernel, typename Args>
+int LaunchCooperative(const Args& args, int grid, size_t smem, cudaStream_t st) {
+  static bool configured[kMaxDevices] = {};
+  const int dev = CurrentDevice();
+  if (!configured[dev]) {
+    CAVS_CUDA(cudaFuncSetAttribute(kKernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kMaxSmem)));
+    configured[dev] = true;
+  }
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(kThreads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeCooperative;   // all CTAs resident, or the launch fails: the barrier needs it
+  attr[0].val.cooperative = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  CAVS_CUDA(cudaLaunchKernelEx(&cfg, kKernel, args));
+  CAVS_LAUNCH_CHECK("narrow levels");
+  return CAVS_OK;
+}
+}  // namespace narrow
+}  // namespace cavs_b200
+#endif
