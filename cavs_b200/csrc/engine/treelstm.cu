@@ -417,8 +417,17 @@ std::vector<NarrowRange> NarrowLevels(const cavs_treelstm* e, const cavs_treelst
     const double per_level = backward ? 16.0 + H / 75.0 : 13.0 + H / 200.0;
     while (begin < bt.n_levels && rows(begin) > 0 && PlanNarrowBf16(H, K, rows(begin), backward).level_us > 0.8 * per_level) ++begin;
     if (begin >= bt.n_levels) return out;
-    const NarrowPlan plan = PlanNarrowBf16(H, K, rows(begin), backward);
-    if (plan.w != 0) out.push_back({begin, bt.n_levels, plan});
+    // Two launches where the levels of one row tile are many: those run backward with one row group, one barrier a level.
+    int split = begin;
+    while (split < bt.n_levels && rows(split) > (K == 1 ? 32 : 16)) ++split;
+    const NarrowPlan wide = PlanNarrowBf16(H, K, rows(begin), backward);
+    if (wide.w == 0) return out;
+    if (split > begin && bt.n_levels - split >= 6 && wide.row_groups > 1) {
+      out.push_back({begin, split, wide});
+      out.push_back({split, bt.n_levels, PlanNarrowBf16(H, K, rows(split), backward)});
+    } else {
+      out.push_back({begin, bt.n_levels, wide});
+    }
     return out;
   }
   while (begin < bt.n_levels && static_cast<double>(rows(begin)) * H * H * (3 + K) > (backward ? 6e7 : 1.2e8)) ++begin;

@@ -32,20 +32,22 @@ __device__ __forceinline__ void StoreAs(float* p, float x) { *p = x; }
 __device__ __forceinline__ void StoreAs(__nv_bfloat16* p, float x) { *p = __float2bfloat16_rn(x); }
 __device__ __forceinline__ void StoreAs(__half* p, float x) { *p = __float2half_rn(x); }
 
-// All CTAs of the grid (launched cooperatively) arrive; false, and *status raised, if that takes too long.
-__device__ __forceinline__ bool GridSync(unsigned* counter, unsigned target, int* status) {
-  __shared__ int s_ok;
+// Grid barrier in two halves, so that requests for data that does not depend on it go out in between.  Arrival releases
+// the CTA's writes (the red is cumulative over what __syncthreads ordered before it); the wait acquires the others', and
+// returns false, *status raised, if they take too long.  All CTAs are resident: the launch is cooperative.
+__device__ __forceinline__ void GridArrive(unsigned* counter) {
   __syncthreads();
-  if (threadIdx.x == 0) {
-    asm volatile("fence.acq_rel.gpu;" ::: "memory");
-    asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(counter) : "memory");
+  if (threadIdx.x == 0) asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(counter) : "memory");
+}
+__device__ __forceinline__ bool GridWait(unsigned* counter, unsigned target, int* status) {
+  __shared__ int s_ok;
+  if (threadIdx.x == kThreads - 32) {   // a warp with few or no rows of its own to request
     int ok = 0;
     for (unsigned it = 0; it < kBarrierPolls; ++it) {
       unsigned v;
       asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(counter) : "memory");
       if (v >= target) { ok = 1; break; }
     }
-    asm volatile("fence.acq_rel.gpu;" ::: "memory");
     if (!ok) atomicExch(status, 1);
     s_ok = ok;
   }
@@ -56,12 +58,15 @@ __device__ __forceinline__ bool GridSync(unsigned* counter, unsigned target, int
 // First phase of a backward level, gate gradients: a thread owns one hidden column and every row_step-th row of each
 // level, so the column sums for the bias gradient stay in its registers.  Expressions and order are CellBwd's.
 // TG: type of the saved gates, TD: type of dA and ZF.
-constexpr int kColBlock = 64, kRowLanes = kThreads / kColBlock;
+// The columns of a CTA: with one row group its own output columns [n0, n0 + w) -- then a level's gradients read only what
+// this CTA wrote into the mailbox, and no grid barrier stands before them; with several, blocks of 64 dealt out over the
+// grid together with strips of rows.
+constexpr int kColBlock = 64;
 template <int K, typename TG, typename TD>
 struct GateGradients {
   static constexpr bool kFast = sizeof(TD) == 2;
-  int j, row0, row_step;
-  bool owner;
+  int j, row0, row_step, cols;
+  bool owner, local;
   float sums[4], wc[kHeadDzPitch];
   // of the next row, everything but its mailbox row
   int ch[K];
@@ -69,11 +74,13 @@ struct GateGradients {
   float gi, go, gu, cown, d_out, gf[K], cch[K];
 
   __device__ __forceinline__ explicit GateGradients(const NarrowBackwardArgs& a) {
-    const int col_blocks = (a.H + kColBlock - 1) / kColBlock, strips = max(1, static_cast<int>(gridDim.x) / col_blocks);
-    const int strip = blockIdx.x / col_blocks;
-    j = (blockIdx.x % col_blocks) * kColBlock + threadIdx.x % kColBlock;
-    row0 = strip * kRowLanes + static_cast<int>(threadIdx.x) / kColBlock;
-    row_step = strips * kRowLanes;
+    local = a.row_groups == 1;
+    cols = local ? a.w : kColBlock;
+    const int col_blocks = (a.H + cols - 1) / cols, strips = local ? 1 : max(1, static_cast<int>(gridDim.x) / col_blocks);
+    const int strip = blockIdx.x / col_blocks, lanes = kThreads / cols;
+    j = (blockIdx.x % col_blocks) * cols + threadIdx.x % cols;
+    row0 = strip * lanes + static_cast<int>(threadIdx.x) / cols;
+    row_step = strips * lanes;
     owner = j < a.H && strip < strips;
 #pragma unroll
     for (int g = 0; g < 4; ++g) sums[g] = 0.0f;
@@ -142,11 +149,11 @@ struct GateGradients {
 #pragma unroll
     for (int g = 0; g < 4; ++g) scratch[g * kThreads + threadIdx.x] = sums[g];
     __syncthreads();
-    if (!owner || threadIdx.x >= kColBlock) return;
+    if (!owner || threadIdx.x >= cols) return;
 #pragma unroll
     for (int g = 0; g < 4; ++g) {
       float acc = 0.0f;
-      for (int r = 0; r < kRowLanes; ++r) acc += scratch[g * kThreads + r * kColBlock + threadIdx.x];
+      for (int r = 0; r < kThreads / cols; ++r) acc += scratch[g * kThreads + r * cols + threadIdx.x];
       a.dB_part[static_cast<size_t>(blockIdx.x) * 4 * a.H + g * a.H + j] += acc;
     }
   }

@@ -48,7 +48,8 @@ __global__ void __launch_bounds__(kThreads, 1) NarrowForwardBf16(const NarrowFor
   const int H = a.H, pk = Pitch(H), steps = (H + 15) / 16;
   bf16* Wb = reinterpret_cast<bf16*>(smem_raw);        // [4 gates i, o, u, f][8 units][pk]
   bf16* At = Wb + 4 * kUnits * pk;                     // [NV][TR][pk]
-  float* red = reinterpret_cast<float*>(At + NV * TR * pk);   // [warps][TR][8][G]
+  // [warps][G][TR][8]: a fragment's float2 stores and the sums' reads fall into all banks
+  float* red = reinterpret_cast<float*>(At + NV * TR * pk);
   const int cg = blockIdx.x % a.col_groups, rg = blockIdx.x / a.col_groups, j0 = cg * kUnits;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int per = (steps + kWarps - 1) / kWarps, step_begin = min(steps, warp * per), step_end = min(steps, step_begin + per);
@@ -160,20 +161,20 @@ __global__ void __launch_bounds__(kThreads, 1) NarrowForwardBf16(const NarrowFor
 #pragma unroll
       for (int m = 0; m < MT; ++m)
 #pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          float* x = red + ((warp * TR + m * 16 + (lane >> 2) + (e >> 1) * 8) * kUnits + (lane & 3) * 2 + (e & 1)) * G;
+        for (int g = 0; g < G; ++g)
 #pragma unroll
-          for (int g = 0; g < G; ++g) x[g] = acc[m][g][e];
-        }
+          for (int e = 0; e < 4; e += 2)
+            *reinterpret_cast<float2*>(red + ((warp * G + g) * TR + m * 16 + (lane >> 2) + e * 4) * kUnits + (lane & 3) * 2) =
+                make_float2(acc[m][g][e], acc[m][g][e + 1]);
       __syncthreads();
       if (pair && prow < rows) {
         float z[G];
 #pragma unroll
         for (int g = 0; g < G; ++g) z[g] = 0.0f;
-        const int used = (steps + per - 1) / per;
-        for (int s = 0; s < used; ++s)
 #pragma unroll
-          for (int g = 0; g < G; ++g) z[g] += red[((s * TR + prow) * kUnits + pu) * G + g];
+        for (int s = 0; s < kWarps; ++s)
+#pragma unroll
+          for (int g = 0; g < G; ++g) z[g] += red[(s * G + g) * TR * kUnits + threadIdx.x];
         const size_t t = t0 + prow;
         const float gi = Sigmoid<true>((in[0] + z[0]) + bi), go = Sigmoid<true>((in[1] + z[1]) + bo), gu = Tanh<true>((in[2] + z[2]) + bu);
         float cc = gi * gu;
@@ -194,8 +195,9 @@ __global__ void __launch_bounds__(kThreads, 1) NarrowForwardBf16(const NarrowFor
     }
     off = end; end = next_end;
     if (l + 1 < a.level_end) {
+      GridArrive(a.barrier);
       prefetch(off, end, rg);
-      if (!GridSync(a.barrier, ++barrier * gridDim.x, a.status)) return;
+      if (!GridWait(a.barrier, ++barrier * gridDim.x, a.status)) return;
     }
   }
 }
@@ -208,7 +210,7 @@ __global__ void __launch_bounds__(kThreads, 1) NarrowBackwardBf16(const NarrowBa
   const int H = a.H, pk = Pitch(H), steps = (H + 15) / 16;
   bf16* Wb = reinterpret_cast<bf16*>(smem_raw);        // [4 blocks i, o, u, f][8 rows n of U][pk]
   bf16* At = Wb + 4 * kUnits * pk;                     // [buffers][TR][pk]
-  float* red = reinterpret_cast<float*>(At + a.buffers * TR * pk);   // [warps][TR][8][1 + K]
+  float* red = reinterpret_cast<float*>(At + a.buffers * TR * pk);   // [warps][1 + K][TR][8]
   const int cg = blockIdx.x % a.col_groups, rg = blockIdx.x / a.col_groups, n0 = cg * kUnits;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int per = (steps + kWarps - 1) / kWarps, step_begin = min(steps, warp * per), step_end = min(steps, step_begin + per);
@@ -232,7 +234,9 @@ __global__ void __launch_bounds__(kThreads, 1) NarrowBackwardBf16(const NarrowBa
   for (int l = a.level_end - 1; l >= a.level_begin; --l) {
     const int next_off = l > a.level_begin ? __ldg(a.level_off + l - 1) : 0;
     gg.Level(a, off, end);
-    if (!GridSync(a.barrier, ++barrier * gridDim.x, a.status)) return;
+    GridArrive(a.barrier);
+    if (l > a.level_begin) gg.Request(a, next_off, off);   // only the mailbox rows are not complete yet
+    if (!GridWait(a.barrier, ++barrier * gridDim.x, a.status)) return;
     const int tiles = (end - off + TR - 1) / TR;
     for (int tile = rg; tile < tiles; tile += a.row_groups) {
       const int t0 = off + tile * TR, rows = min(TR, end - t0);
@@ -291,30 +295,32 @@ __global__ void __launch_bounds__(kThreads, 1) NarrowBackwardBf16(const NarrowBa
 #pragma unroll
       for (int m = 0; m < MT; ++m)
 #pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          float* x = red + ((warp * TR + m * 16 + (lane >> 2) + (e >> 1) * 8) * kUnits + (lane & 3) * 2 + (e & 1)) * (1 + K);
-          x[0] = ds[m][e];
+        for (int e = 0; e < 4; e += 2) {
+          float* x = red + (warp * (1 + K) * TR + m * 16 + (lane >> 2) + e * 4) * kUnits + (lane & 3) * 2;
+          *reinterpret_cast<float2*>(x) = make_float2(ds[m][e], ds[m][e + 1]);
 #pragma unroll
-          for (int c = 0; c < K; ++c) x[1 + c] = dq[c][m][e];
+          for (int c = 0; c < K; ++c) *reinterpret_cast<float2*>(x + (1 + c) * TR * kUnits) = make_float2(dq[c][m][e], dq[c][m][e + 1]);
         }
       __syncthreads();
       if (pair) {
         float z[1 + K];
 #pragma unroll
         for (int c = 0; c <= K; ++c) z[c] = 0.0f;
-        const int used = (steps + per - 1) / per;
-        for (int s = 0; s < used; ++s)
 #pragma unroll
-          for (int c = 0; c <= K; ++c) z[c] += red[((s * TR + prow) * kUnits + pu) * (1 + K) + c];
+        for (int s = 0; s < kWarps; ++s)
+#pragma unroll
+          for (int c = 0; c <= K; ++c) z[c] += red[(s * (1 + K) + c) * TR * kUnits + threadIdx.x];
 #pragma unroll
         for (int c = 0; c < K; ++c)
           if (chn[c] >= 0) a.mailbox[static_cast<size_t>(chn[c]) * 2 * H + col] = z[0] + z[1 + c];
       }
     }
     end = off; off = next_off;
-    if (l > a.level_begin) {
-      gg.Request(a, off, end);   // only the mailbox waits for the barrier
-      if (!GridSync(a.barrier, ++barrier * gridDim.x, a.status)) return;
+    if (gg.local) {
+      __syncthreads();   // the next level's rows of these columns were written by this CTA
+    } else if (l > a.level_begin) {
+      GridArrive(a.barrier);
+      if (!GridWait(a.barrier, ++barrier * gridDim.x, a.status)) return;
     }
   }
   gg.FoldSums(a, red);
@@ -334,11 +340,14 @@ NarrowPlan PlanNarrowBf16(int H, int K, int rows, bool backward) {
   if (p.smem > kMaxSmem) return NarrowPlan();
   p.w = kUnits;
   p.col_groups = cols;
-  p.row_groups = std::min(SmCount() / cols, tiles);
-  // us: barriers and dependent round trips, a tile's own round trips, and the rows every CTA pulls out of L2
-  const double mine = (tiles + p.row_groups - 1) / p.row_groups;
-  const double bytes = static_cast<double>(cols) * rows * H * (backward ? 2.0 * (3 + K) : 4.0 * K);
-  p.level_us = (backward ? 6.0 : 3.5) + 1.5 * mine + bytes / 5e6;
+  // us: barriers and dependent round trips, a tile's own round trips, and the rows every CTA pulls out of L2.  Backward
+  // with one row group has one barrier per level instead of two, but every CTA takes every row.
+  for (int groups : {1, std::min(SmCount() / cols, tiles)}) {
+    const double mine = (tiles + groups - 1) / groups;
+    const double bytes = static_cast<double>(cols) * rows * H * (backward ? 2.0 * (3 + K) : 4.0 * K);
+    const double us = (backward ? (groups > 1 ? 7.0 : 4.5) : 3.5) + (backward ? 2.5 : 1.5) * mine + std::max(bytes / 5e6, bytes / cols / groups / 0.1e6);
+    if (p.row_groups == 0 || us < p.level_us) { p.row_groups = groups; p.level_us = us; }
+  }
   return p;
 }
 

@@ -119,7 +119,7 @@ __device__ __forceinline__ void FwdProducts(const float* At, int p, const float4
 #pragma unroll
   for (int r = 0; r < RPT; ++r)
 #pragma unroll
-    for (int g = 0; g < G; ++g) red[(((lane >> 2) + r * 8) * w + unit) * G + g] = acc[r][g];
+    for (int g = 0; g < G; ++g) red[(g * TR + (lane >> 2) + r * 8) * w + unit] = acc[r][g];
 }
 
 template <int K, int V>
@@ -130,7 +130,7 @@ __global__ void __launch_bounds__(kThreads, 1) NarrowForward(const NarrowForward
   const int H = a.H, w = a.w, hk = Pad4(H), p = Pitch(hk);
   float4* Ub = reinterpret_cast<float4*>(smem);                 // [hk][w]: i, o, u, f columns of a unit
   float* At0 = smem + static_cast<size_t>(hk) * w * 4;           // [buffers][K][TR][p]
-  float* red = At0 + a.buffers * K * TR * p;                                  // [k slices][TR][w][G]
+  float* red = At0 + a.buffers * K * TR * p;                                  // [k slices][G][TR][w]
   const int cg = blockIdx.x % a.col_groups, rg = blockIdx.x / a.col_groups, j0 = cg * w;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int unit_warps = w / 4, slices = kWarps / unit_warps;
@@ -220,9 +220,10 @@ __global__ void __launch_bounds__(kThreads, 1) NarrowForward(const NarrowForward
         float z[G];
 #pragma unroll
         for (int g = 0; g < G; ++g) z[g] = 0.0f;
+#pragma unroll 4
         for (int s = 0; s < slices; ++s)
 #pragma unroll
-          for (int g = 0; g < G; ++g) z[g] += red[((s * TR + prow) * w + threadIdx.x % w) * G + g];
+          for (int g = 0; g < G; ++g) z[g] += red[(s * G + g) * TR * w + threadIdx.x];
         const size_t t = t0 + prow;
         const float gi = Sigmoid<false>((x[0] + z[0]) + bi), go = Sigmoid<false>((x[1] + z[1]) + bo), gu = tanhf((x[2] + z[2]) + bu);
         float cc = gi * gu, sum = 0.0f;
@@ -248,8 +249,9 @@ __global__ void __launch_bounds__(kThreads, 1) NarrowForward(const NarrowForward
     }
     off = end; end = next_end;
     if (l + 1 < a.level_end) {
+      GridArrive(a.barrier);
       prefetch(off, end, rg);
-      if (!GridSync(a.barrier, ++barrier * gridDim.x, a.status)) return;
+      if (!GridWait(a.barrier, ++barrier * gridDim.x, a.status)) return;
     }
   }
 }
@@ -333,19 +335,20 @@ __device__ __forceinline__ void BwdTile(const NarrowBackwardArgs& a, const float
   for (int r = 0; r < RPT; ++r)
 #pragma unroll
     for (int n = 0; n < NPT; ++n) {
-      float* x = my_red + (((lane >> 2) + r * 8) * w + unit + n * 4) * (1 + K);
+      float* x = my_red + ((lane >> 2) + r * 8) * w + unit + n * 4;
       x[0] = ds[r][n];
 #pragma unroll
-      for (int c = 0; c < K; ++c) x[1 + c] = dq[c][r][n];
+      for (int c = 0; c < K; ++c) x[(1 + c) * TR * w] = dq[c][r][n];
     }
   __syncthreads();
   if (pair) {
     float z[1 + K];
 #pragma unroll
     for (int c = 0; c <= K; ++c) z[c] = 0.0f;
+#pragma unroll 4
     for (int s = 0; s < slices; ++s)
 #pragma unroll
-      for (int c = 0; c <= K; ++c) z[c] += red[((s * TR + prow) * w + threadIdx.x % w) * (1 + K) + c];
+      for (int c = 0; c <= K; ++c) z[c] += red[(s * (1 + K) + c) * TR * w + threadIdx.x];
 #pragma unroll
     for (int c = 0; c < K; ++c)
       if (chn[c] >= 0) a.mailbox[static_cast<size_t>(chn[c]) * 2 * H + col] = z[0] + z[1 + c];
@@ -359,7 +362,7 @@ __global__ void __launch_bounds__(kThreads, 1) NarrowBackward(const NarrowBackwa
   const int H = a.H, w = a.w, hk = Pad4(H), p = Pitch(hk), pw = Pitch(4 * hk);
   float* Wt = smem;                        // [w][pw]: row n of U_iou (three blocks) and U_f, each block padded to hk
   float* At = Wt + static_cast<size_t>(w) * pw;   // [buffers][TR][p]
-  float* red = At + static_cast<size_t>(a.buffers) * TR * p;   // [k slices][TR][w][1 + K]
+  float* red = At + static_cast<size_t>(a.buffers) * TR * p;   // [k slices][1 + K][TR][w]
   const int cg = blockIdx.x % a.col_groups, rg = blockIdx.x / a.col_groups, n0 = cg * w;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int unit_warps = w / (4 * NPT), slices = kWarps / unit_warps;
@@ -381,7 +384,9 @@ __global__ void __launch_bounds__(kThreads, 1) NarrowBackward(const NarrowBackwa
   for (int l = a.level_end - 1; l >= a.level_begin; --l) {
     const int next_off = l > a.level_begin ? __ldg(a.level_off + l - 1) : 0;
     gg.Level(a, off, end);
-    if (!GridSync(a.barrier, ++barrier * gridDim.x, a.status)) return;
+    GridArrive(a.barrier);
+    if (l > a.level_begin) gg.Request(a, next_off, off);   // only the mailbox rows are not complete yet
+    if (!GridWait(a.barrier, ++barrier * gridDim.x, a.status)) return;
     const int tiles = (end - off + TR - 1) / TR;
     for (int tile = rg; tile < tiles; tile += a.row_groups) {
       const int t0 = off + tile * TR, rows = min(TR, end - t0);
@@ -389,9 +394,11 @@ __global__ void __launch_bounds__(kThreads, 1) NarrowBackward(const NarrowBackwa
       else BwdTile<K, V, NPT, TR / 8>(a, Wt, pw, At, p, red, t0, rows, n0, unit, slice, slices, k4_begin, k4_end);
     }
     end = off; off = next_off;
-    if (l > a.level_begin) {
-      gg.Request(a, off, end);   // only the mailbox waits for the barrier
-      if (!GridSync(a.barrier, ++barrier * gridDim.x, a.status)) return;
+    if (gg.local) {
+      __syncthreads();   // the next level's rows of these columns were written by this CTA
+    } else if (l > a.level_begin) {
+      GridArrive(a.barrier);
+      if (!GridWait(a.barrier, ++barrier * gridDim.x, a.status)) return;
     }
   }
   gg.FoldSums(a, red);
@@ -430,13 +437,14 @@ NarrowPlan PlanNarrowF32(int H, int K, int rows, bool backward) {
   const int tr = K <= 2 ? 32 : 16;
   const int tiles = (rows + tr - 1) / tr;
   double best_cost = 0.0;
-  for (int w : {4, 8, 16}) {
+  for (int w : {4, 8, 16})
+   for (int groups : {1, 2}) {   // one row group, or as many as fit
     const int cols = (H + w - 1) / w;
     if (cols > SmCount()) continue;
     NarrowPlan p;
     p.w = w;
     p.col_groups = cols;
-    p.row_groups = std::min(SmCount() / cols, tiles);
+    p.row_groups = groups == 1 ? 1 : std::min(SmCount() / cols, tiles);
     p.buffers = 3 + K;
     if (backward) {
       while (p.buffers > 0 && BackwardSmem(H, K, w, p.buffers) > kMaxSmem) --p.buffers;
@@ -453,7 +461,8 @@ NarrowPlan PlanNarrowF32(int H, int K, int rows, bool backward) {
     const double rate = backward ? (w >= 8 ? 0.15 : 0.11) : (w >= 8 ? 0.28 : 0.2);
     const double load = backward ? 0.5 * (3 + K) : 1.0, work = static_cast<double>(tr) * w * H * (3 + K) / (128.0 * rate * 1900.0);
     const int mine = (tiles + p.row_groups - 1) / p.row_groups;
-    const double cost = p.buffers > 1 ? load + mine * std::max(work, 0.6 * load) : mine * (load + work);
+    // (backward: the second barrier, which one row group does without)
+    const double cost = (p.buffers > 1 ? load + mine * std::max(work, 0.6 * load) : mine * (load + work)) + (backward && p.row_groups > 1 ? 2.5 : 0.0);
     if (best.w == 0 || cost < best_cost) { best = p; best_cost = cost; }
   }
   best.level_us = 3.0 + best_cost;
