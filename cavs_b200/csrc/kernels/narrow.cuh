@@ -9,6 +9,7 @@
 #include <cstdint>
 
 #include "abi_common.h"
+#include "kernels/bulk.cuh"
 #include "kernels/cell.h"
 #include "kernels/launch.h"
 #include "kernels/narrow.h"
@@ -54,6 +55,52 @@ __device__ __forceinline__ bool GridWait(unsigned* counter, unsigned target, int
   __syncthreads();
   return s_ok != 0;
 }
+
+// Rows that arrive in shared memory by bulk copies, one mbarrier per buffer.  A row is one copy: with nearly all of an SM's
+// memory given to shared memory, per-thread asynchronous copies have so little of L1 left to fly through that issuing
+// 128 KB of them took 6.1 k clocks.  Sources were written by other SMs' ordinary stores before the grid barrier, hence the
+// proxy fence of the issuing lanes.
+template <int kBuffers>
+struct BulkRows {
+  uint64_t* bars;
+  uint32_t phases = 0;
+  bool ok = true;
+  __device__ __forceinline__ void Init(uint64_t* shared, int arrivals) {   // followed by a __syncthreads of the caller
+    bars = shared;
+    if (threadIdx.x == 0) {
+      for (int i = 0; i < kBuffers; ++i) bulk::MbarInit(bulk::SmemAddr(bars + i), arrivals);
+      bulk::FenceMbarInit();
+    }
+  }
+  // By one warp: lane r copies `bytes` from src (nullptr: nothing) to dst + r * pitch; one arrival.
+  __device__ __forceinline__ void Copy(int buf, uint32_t dst, uint32_t pitch, const void* src, uint32_t bytes) {
+    const int lane = threadIdx.x & 31;
+    const unsigned live = __ballot_sync(0xffffffffu, src != nullptr);
+    const uint32_t bar = bulk::SmemAddr(bars + buf);
+    asm volatile("fence.proxy.async;" ::: "memory");
+    if (lane == 0) bulk::MbarExpectTx(bar, __popc(live) * bytes);
+    __syncwarp();
+    if (src != nullptr) bulk::Load(dst + lane * pitch, src, bytes, bar);
+  }
+  // By all threads; after one expired wait nothing is waited for any more (and *status is raised).
+  __device__ __forceinline__ void Wait(int buf, int* status) {
+    if (ok) {
+      const uint32_t bar = bulk::SmemAddr(bars + buf), parity = (phases >> buf) & 1;
+      ok = false;
+      for (uint32_t it = 0; it < (1u << 18) && !ok; ++it) {
+        uint32_t done;
+        asm volatile(
+            "{\n\t.reg .pred p;\n\t"
+            "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, 1000;\n\t"
+            "selp.u32 %0, 1, 0, p;\n\t}"
+            : "=r"(done) : "r"(bar), "r"(parity) : "memory");
+        ok = done != 0;
+      }
+      if (!ok) atomicExch(status, 1);
+    }
+    phases ^= 1u << buf;
+  }
+};
 
 // First phase of a backward level, gate gradients: a thread owns one hidden column and every row_step-th row of each
 // level, so the column sums for the bias gradient stay in its registers.  Expressions and order are CellBwd's.

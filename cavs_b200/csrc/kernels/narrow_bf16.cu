@@ -223,6 +223,9 @@ __global__ void __launch_bounds__(kThreads, 1) NarrowBackwardBf16(const NarrowBa
     *reinterpret_cast<uint4*>(Wb + row * pk + k) = __ldg(reinterpret_cast<const uint4*>(u));
   }
   GateGradients<K, __half, bf16> gg(a);
+  __shared__ uint64_t s_full[G];
+  BulkRows<G> ring;
+  ring.Init(s_full, 1);
   __syncthreads();
   const uint32_t b_addr = SmemAddr(Wb + (lane & 7) * pk + ((lane >> 3) & 1) * 8);
   const uint32_t a_addr = SmemAddr(At + (lane & 15) * pk + (lane >> 4) * 8);
@@ -244,16 +247,13 @@ __global__ void __launch_bounds__(kThreads, 1) NarrowBackwardBf16(const NarrowBa
       int chn[K];
 #pragma unroll
       for (int c = 0; c < K; ++c) chn[c] = pair ? __ldg(a.child + static_cast<size_t>(c) * a.n_total + t0 + prow) : -1;
-      // vectors zi, zo, zu, zf_0.. through a ring of buffers; rows past the level's end keep what the buffer held
+      // vectors zi, zo, zu, zf_0.. through a ring of buffers, one warp's copies each; rows past the level's end keep what the
+      // buffer held
       auto load = [&](int q) {
-        bf16* dst = At + (q % a.buffers) * TR * pk;
-        for (int r = threadIdx.x >> 6; r < rows; r += kThreads / 64) {
-          const size_t t = t0 + r;
-          const bf16* s = q < 3 ? static_cast<const bf16*>(a.dA) + t * 4 * H + q * H : static_cast<const bf16*>(a.ZF) + (t * K + q - 3) * H;
-          for (int j = (threadIdx.x & 63) * 8; j < H; j += 512)
-            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(SmemAddr(dst + r * pk + j)), "l"(s + j) : "memory");
-        }
-        asm volatile("cp.async.commit_group;" ::: "memory");
+        if (warp != q) return;
+        const size_t t = t0 + lane;
+        const bf16* s = q < 3 ? static_cast<const bf16*>(a.dA) + t * 4 * H + q * H : static_cast<const bf16*>(a.ZF) + (t * K + q - 3) * H;
+        ring.Copy(q % a.buffers, SmemAddr(At + (q % a.buffers) * TR * pk), pk * 2, lane < rows ? s : nullptr, H * 2);
       };
       float ds[MT][4], dq[K][MT][4];
 #pragma unroll
@@ -269,12 +269,7 @@ __global__ void __launch_bounds__(kThreads, 1) NarrowBackwardBf16(const NarrowBa
       for (int q = 0; q < ahead; ++q) load(q);
 #pragma unroll
       for (int q = 0; q < G; ++q) {
-        const int pending = min(a.buffers - 1, G - 1 - q);   // groups requested after q's
-        if (pending >= 3) asm volatile("cp.async.wait_group 3;" ::: "memory");
-        else if (pending == 2) asm volatile("cp.async.wait_group 2;" ::: "memory");
-        else if (pending == 1) asm volatile("cp.async.wait_group 1;" ::: "memory");
-        else asm volatile("cp.async.wait_group 0;" ::: "memory");
-        __syncthreads();
+        ring.Wait(q % a.buffers, a.status);
         for (int st = step_begin; st < step_end; ++st) {
           uint32_t b[2];
           LdMatrix2(b, b_addr + min(q, 3) * kUnits * pk * 2 + st * 32);

@@ -35,50 +35,45 @@ __host__ __device__ inline int Pad4(int x) { return (x + 3) & ~3; }
 // Row pitch with which eight consecutive rows start in eight different groups of four banks.
 __host__ __device__ inline int Pitch(int x) { return ((x + 31) & ~31) + 4; }
 
-// rows x H floats (row r at src(r), nullptr: zeros) into dst (row pitch p), columns up to Pad4(H) zeroed.  Rows of whole
-// 16-byte words are copied asynchronously (the caller waits for the group), others through registers, eight loads in
-// flight per thread.  Both bypass L1.
+// rows x H floats (row r at src(r), nullptr: zeros) into dst (row pitch p), columns up to Pad4(H) zeroed, through registers
+// with L1 bypassed, eight loads in flight per thread: widths whose rows are no whole 16-byte words.
 template <int V, typename F>
 __device__ __forceinline__ void LoadRows(float* dst, int p, int rows, int H, F src) {
   const int hv = Pad4(H) / V, tpr = hv <= 32 ? 32 : hv <= 64 ? 64 : 128, lane = threadIdx.x & (tpr - 1), step = kThreads / tpr;
-  if constexpr (V == 4) {
-    for (int r = threadIdx.x / tpr; r < rows; r += step) {
-      const float* s = src(r);
-      const uint32_t d = static_cast<uint32_t>(__cvta_generic_to_shared(dst + r * p));
-      for (int j = lane; j < hv; j += tpr) {
-        if (s != nullptr)
-          asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d + j * 16), "l"(s + j * 4) : "memory");
-        else
-          *reinterpret_cast<float4*>(dst + r * p + j * 4) = make_float4(0.f, 0.f, 0.f, 0.f);
-      }
-    }
-  } else {
-    constexpr int kBatch = 8;
-    for (int r0 = threadIdx.x / tpr; r0 < rows; r0 += step * kBatch)
-      for (int j = lane; j < hv; j += tpr) {
-        float v[kBatch][V];
+  constexpr int kBatch = 8;
+  for (int r0 = threadIdx.x / tpr; r0 < rows; r0 += step * kBatch)
+    for (int j = lane; j < hv; j += tpr) {
+      float v[kBatch][V];
 #pragma unroll
-        for (int u = 0; u < kBatch; ++u) {
-          const int r = r0 + u * step;
-          const float* s = r < rows && j * V < H ? src(r) : nullptr;
+      for (int u = 0; u < kBatch; ++u) {
+        const int r = r0 + u * step;
+        const float* s = r < rows && j * V < H ? src(r) : nullptr;
 #pragma unroll
-          for (int e = 0; e < V; ++e) v[u][e] = 0.0f;
-          if (s != nullptr) {
-            if constexpr (V == 2) { const float2 t = __ldcg(reinterpret_cast<const float2*>(s) + j); v[u][0] = t.x; v[u][1] = t.y; }
-            else v[u][0] = __ldcg(s + j);
-          }
+        for (int e = 0; e < V; ++e) v[u][e] = 0.0f;
+        if (s != nullptr) {
+          if constexpr (V == 2) { const float2 t = __ldcg(reinterpret_cast<const float2*>(s) + j); v[u][0] = t.x; v[u][1] = t.y; }
+          else v[u][0] = __ldcg(s + j);
         }
-#pragma unroll
-        for (int u = 0; u < kBatch; ++u)
-          if (r0 + u * step < rows) {
-#pragma unroll
-            for (int e = 0; e < V; ++e) dst[(r0 + u * step) * p + j * V + e] = v[u][e];
-          }
       }
-  }
+#pragma unroll
+      for (int u = 0; u < kBatch; ++u)
+        if (r0 + u * step < rows) {
+#pragma unroll
+          for (int e = 0; e < V; ++e) dst[(r0 + u * step) * p + j * V + e] = v[u][e];
+        }
+    }
 }
-__device__ __forceinline__ void CommitRows() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-__device__ __forceinline__ void WaitRows() { asm volatile("cp.async.wait_group 0;" ::: "memory"); }
+// The same by one warp with bulk copies (H a multiple of 4), lane r taking row r of up to 32; arrives once on the buffer.
+template <int kBuffers, typename F>
+__device__ __forceinline__ void CopyRows(BulkRows<kBuffers>& ring, int buf, float* dst, int p, int rows, int H, F src) {
+  const int lane = threadIdx.x & 31;
+  const float* s = lane < rows ? src(lane) : nullptr;
+  unsigned empty = __ballot_sync(0xffffffffu, lane < rows && s == nullptr);
+  for (; empty != 0; empty &= empty - 1)   // no child there: zeros
+    for (int j = lane * 4; j < H; j += 128) *reinterpret_cast<float4*>(dst + (__ffs(empty) - 1) * p + j) = make_float4(0.f, 0.f, 0.f, 0.f);
+  __syncwarp();
+  ring.Copy(buf, static_cast<uint32_t>(__cvta_generic_to_shared(dst)), p * 4, s, H * 4);
+}
 
 // ---- forward ----
 template <int K, int RPT>
@@ -148,6 +143,9 @@ __global__ void __launch_bounds__(kThreads, 1) NarrowForward(const NarrowForward
   float bi = 0.f, bf = 0.f, bu = 0.f, bo = 0.f;
   if (pair) { bi = a.bias[pj]; bf = a.bias[H + pj]; bu = a.bias[2 * H + pj]; bo = a.bias[3 * H + pj]; }
 
+  __shared__ uint64_t s_full[2];
+  BulkRows<2> ring;
+  ring.Init(s_full, K);
   int off = __ldg(a.level_off + a.level_begin), end = __ldg(a.level_off + a.level_begin + 1);
   unsigned barrier = 0;
   // What the next tile needs beside the previous level's states is requested before the barrier.
@@ -172,12 +170,17 @@ __global__ void __launch_bounds__(kThreads, 1) NarrowForward(const NarrowForward
     auto load_rows = [&](int tile, int buf) {
       const int live = min(TR, (end - off - tile * TR + 7) & ~7);   // whole groups of eight rows
 #pragma unroll
-      for (int c = 0; c < K; ++c)
-        LoadRows<V>(At0 + (buf * K + c) * TR * p, p, live, H, [&](int r) {
+      for (int c = 0; c < K; ++c) {
+        auto row = [&](int r) -> const float* {
           const int ch = s_child[buf][c][r];
           return ch >= 0 ? a.state + static_cast<size_t>(ch) * 2 * H : nullptr;
-        });
-      CommitRows();
+        };
+        if constexpr (V == 4) {
+          if (warp == c) CopyRows(ring, buf, At0 + (buf * K + c) * TR * p, p, live, H, row);
+        } else {
+          LoadRows<V>(At0 + (buf * K + c) * TR * p, p, live, H, row);
+        }
+      }
     };
     int buf = 0;
     for (int tile = rg; tile < tiles; tile += a.row_groups, buf ^= 1) {
@@ -207,7 +210,7 @@ __global__ void __launch_bounds__(kThreads, 1) NarrowForward(const NarrowForward
         prefetch(off, end, tile + a.row_groups);
         if (a.buffers == 2 && threadIdx.x < K * TR) s_child[buf ^ 1][threadIdx.x / TR][threadIdx.x % TR] = child;
       }
-      WaitRows();
+      if constexpr (V == 4) ring.Wait(nbuf, a.status);
       __syncthreads();
       if (more && a.buffers == 2) load_rows(tile + a.row_groups, buf ^ 1);   // arrives under this tile's products
       const float* At = At0 + nbuf * K * TR * p;
@@ -282,7 +285,7 @@ __device__ __forceinline__ void BwdProducts(float (&acc)[RPT][NPT], const float*
 
 // One tile of the second phase: d(h) of the children of rows [t0, t0 + rows), this CTA's columns.
 template <int K, int V, int NPT, int RPT>
-__device__ __forceinline__ void BwdTile(const NarrowBackwardArgs& a, const float* Wt, int pw, float* At, int p, float* red, int t0, int rows, int n0,
+__device__ __forceinline__ void BwdTile(const NarrowBackwardArgs& a, const float* Wt, int pw, float* At, int p, float* red, BulkRows<3 + K>& ring, int t0, int rows, int n0,
                                         int unit, int slice, int slices, int k4_begin, int k4_end) {
   constexpr int TR = TileRows<K>(), G = 3 + K;
   const int H = a.H, w = a.w, hk = Pad4(H), lane = threadIdx.x & 31;
@@ -302,25 +305,25 @@ __device__ __forceinline__ void BwdTile(const NarrowBackwardArgs& a, const float
     }
   // Vectors zi, zo, zu, zf_0.. pass through a ring of buffers: as many as fit are requested ahead of their products.
   auto load = [&](int q) {
-    LoadRows<V>(At + (q % a.buffers) * TR * p, p, RPT * 8, H, [&](int r) -> const float* {
+    auto row = [&](int r) -> const float* {
       if (r >= rows) return nullptr;
       const size_t t = t0 + r;
       return q < 3 ? static_cast<const float*>(a.dA) + t * 4 * H + q * H : static_cast<const float*>(a.ZF) + (t * K + q - 3) * H;
-    });
-    CommitRows();
+    };
+    float* dst = At + (q % a.buffers) * TR * p;
+    if constexpr (V == 4) {
+      if (static_cast<int>(threadIdx.x >> 5) == q) CopyRows(ring, q % a.buffers, dst, p, rows, H, row);
+    } else {
+      LoadRows<V>(dst, p, RPT * 8, H, row);
+    }
   };
   __syncthreads();   // readers of the buffers and of the sums are done
   const int ahead = min(a.buffers, G);
   for (int q = 0; q < ahead; ++q) load(q);
 #pragma unroll
   for (int q = 0; q < G; ++q) {
-    // groups requested after q's: those of q + 1 .. ahead - 1, plus one for each buffer already reused
-    const int pending = min(a.buffers - 1, G - 1 - q);
-    if (pending >= 3) asm volatile("cp.async.wait_group 3;" ::: "memory");
-    else if (pending == 2) asm volatile("cp.async.wait_group 2;" ::: "memory");
-    else if (pending == 1) asm volatile("cp.async.wait_group 1;" ::: "memory");
-    else asm volatile("cp.async.wait_group 0;" ::: "memory");
-    __syncthreads();
+    if constexpr (V == 4) ring.Wait(q % a.buffers, a.status);
+    else __syncthreads();
     const float* buf = At + (q % a.buffers) * TR * p;
     const float* wt = Wt + unit * pw + min(q, 3) * hk;
     if (q < 3) BwdProducts<RPT, NPT>(ds, buf, p, wt, pw, k4_begin, k4_end, lane);
@@ -376,6 +379,9 @@ __global__ void __launch_bounds__(kThreads, 1) NarrowBackward(const NarrowBackwa
       Wt[n * pw + i] = v;
     }
   GateGradients<K, float, float> gg(a);
+  __shared__ uint64_t s_full[3 + K];
+  BulkRows<3 + K> ring;
+  ring.Init(s_full, 1);
   __syncthreads();
 
   int end = __ldg(a.level_off + a.level_end), off = __ldg(a.level_off + a.level_end - 1);
@@ -390,8 +396,8 @@ __global__ void __launch_bounds__(kThreads, 1) NarrowBackward(const NarrowBackwa
     const int tiles = (end - off + TR - 1) / TR;
     for (int tile = rg; tile < tiles; tile += a.row_groups) {
       const int t0 = off + tile * TR, rows = min(TR, end - t0);
-      if (rows <= 8) BwdTile<K, V, NPT, 1>(a, Wt, pw, At, p, red, t0, rows, n0, unit, slice, slices, k4_begin, k4_end);
-      else BwdTile<K, V, NPT, TR / 8>(a, Wt, pw, At, p, red, t0, rows, n0, unit, slice, slices, k4_begin, k4_end);
+      if (rows <= 8) BwdTile<K, V, NPT, 1>(a, Wt, pw, At, p, red, ring, t0, rows, n0, unit, slice, slices, k4_begin, k4_end);
+      else BwdTile<K, V, NPT, TR / 8>(a, Wt, pw, At, p, red, ring, t0, rows, n0, unit, slice, slices, k4_begin, k4_end);
     }
     end = off; off = next_off;
     if (gg.local) {
