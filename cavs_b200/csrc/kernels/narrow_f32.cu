@@ -6,8 +6,7 @@
 // per level and direction however few rows it has.  Here a CTA keeps its slice of the recurrent weights in shared memory
 // for all levels, a tile of rows is gathered, multiplied, finished and stored by the CTA that owns its columns, and a
 // level costs a barrier, a few dependent round trips to L2 and its arithmetic (FFMA in fp32, k ascending within a
-// k slice).  Twenty rows, H = 200, one child slot: 25 -> 4.9 us forward, 27 -> 10.8 us backward with two barriers per
-// level.  Wide levels stay with the tensor-core products: the multiply-adds here are bound by shared-memory reads (146
+// k slice).  Twenty rows, H = 200, one child slot: 25 -> 4.9 us forward, 27 -> 8 us backward.  Wide levels stay with the tensor-core products: the multiply-adds here are bound by shared-memory reads (146
 // rows, H = 512: 20 us forward, 53 backward).
 //
 // Forward: CTA (column group, row group) owns w hidden units with all four gates; a warp's lanes are 8 rows x 4 units,
