@@ -75,6 +75,16 @@ __device__ __forceinline__ Vec<V> LoadF(const __half* p) {
   }
   return r;
 }
+// A parameter row (bias, classifier) wherever it starts: the blocks of the flat parameter buffer lie behind an embedding
+// table of any size.  Read once per thread, so the test costs nothing beside the row loop.
+template <int V>
+__device__ __forceinline__ Vec<V> LoadParam(const float* p) {
+  if ((reinterpret_cast<uintptr_t>(p) & (4 * V - 1)) == 0) return LoadF<V>(p);
+  Vec<V> r;
+#pragma unroll
+  for (int e = 0; e < V; ++e) r.v[e] = p[e];
+  return r;
+}
 template <int V>
 __device__ __forceinline__ Vec<V> Zero() { Vec<V> r; for (int i = 0; i < V; ++i) r.v[i] = 0.0f; return r; }
 
@@ -378,7 +388,7 @@ CellBwd(T* __restrict__ dA, T* __restrict__ ZF, float* __restrict__ mailbox, flo
         const size_t ar = a_row ? static_cast<size_t>(__ldg(a_row + t)) : t;
         const T* a = A + ar * 4 * H + j;
         const Vec<V> ai = LoadF<V>(a), ao = LoadF<V>(a + H), au = LoadF<V>(a + 2 * H);
-        const Vec<V> bi = LoadF<V>(bias + j), bu = LoadF<V>(bias + 2 * H + j), bo = LoadF<V>(bias + 3 * H + j);
+        const Vec<V> bi = LoadParam<V>(bias + j), bu = LoadParam<V>(bias + 2 * H + j), bo = LoadParam<V>(bias + 3 * H + j);
 #pragma unroll
         for (int e = 0; e < V; ++e) {
           gi.v[e] = SigmoidT<sizeof(T) == 2>((ai.v[e] + 0.0f) + bi.v[e]);
@@ -981,7 +991,7 @@ TokenGradChunks(float* __restrict__ partial, T* __restrict__ out, const int32_t*
   }
   for (int j = threadIdx.x * V; j < H; j += kThreads * V) {
     const Vec<V> ai = LoadF<V>(a + j), ao = LoadF<V>(a + H + j), au = LoadF<V>(a + 2 * H + j);
-    const Vec<V> bi = LoadF<V>(lg.bias + j), bu = LoadF<V>(lg.bias + 2 * H + j), bo = LoadF<V>(lg.bias + 3 * H + j);
+    const Vec<V> bi = LoadParam<V>(lg.bias + j), bu = LoadParam<V>(lg.bias + 2 * H + j), bo = LoadParam<V>(lg.bias + 3 * H + j);
     Vec<V> gi, go, gu, th;
 #pragma unroll
     for (int e = 0; e < V; ++e) {
@@ -995,7 +1005,7 @@ TokenGradChunks(float* __restrict__ partial, T* __restrict__ out, const int32_t*
     Vec<V> wc[kHeadDzPitch];
     if (by_dz) {
 #pragma unroll
-      for (int c = 0; c < kHeadDzPitch; ++c) wc[c] = c < lg.C ? LoadF<V>(lg.Wc + static_cast<size_t>(c) * H + j) : Zero<V>();
+      for (int c = 0; c < kHeadDzPitch; ++c) wc[c] = c < lg.C ? LoadParam<V>(lg.Wc + static_cast<size_t>(c) * H + j) : Zero<V>();
     }
     Vec<V> si = Zero<V>(), so = Zero<V>(), su = Zero<V>();
     // Rows in pairs: the loads of a pair are issued together (a chunk of a frequent token is a long
@@ -1117,9 +1127,6 @@ LinkSumChunks(float* __restrict__ partial, T* __restrict__ out, const int32_t* _
   }
 }
 
-int VecWidth(int H) { return H % 4 == 0 ? 4 : (H % 2 == 0 ? 2 : 1); }
-
-
 #define DISPATCH_KV(K_, V_, ...)                                             \
   do {                                                                        \
     const int _k = (K_), _v = (V_);                                           \
@@ -1179,7 +1186,7 @@ int LaunchCellFwd(float* state, void* gates, const void* A, const void* P, const
   CAVS_REQUIRE(tok_base < 0 || (!leaf && P != nullptr), CAVS_ERR_BAD_ARG, "treelstm_cell_fwd: per-token products apply to an internal level");
   if (int rc = CheckCommon("treelstm_cell_fwd", rows, H, K)) return rc;
   if (rows == 0) return CAVS_OK;
-  const int v = VecWidth(H);
+  const int v = VecWidth(H, bias);
   // The by-token level of the bf16 configuration streams its rows through shared memory (CellFwdTokStream).
   static const bool stream_ok = [] { const char* e = std::getenv("CAVS_CELL_FWD_STREAM"); return !(e != nullptr && e[0] == '0'); }();
   if (stream_ok && preact_bf16 && tok_base >= 0 && !leaf && H % 8 == 0 && H / 4 <= kBwdConsumers && H / 4 >= 128) {
@@ -1328,6 +1335,8 @@ int LaunchTokenGradChunks(float* partial, void* out, bool bf16, const int32_t* c
   CAVS_REQUIRE(partial && out && chunk_out && dA && A && order && chunk_off && chunk_seg && mailbox && bias &&
                    ((dz || ptok) ? (Wc && C >= 1 && C <= kHeadDzPitch && (!ptok || hist)) : dOut != nullptr),
                CAVS_ERR_BAD_ARG, "token_grad_chunks: null pointer");
+  CAVS_REQUIRE(ptok == nullptr || ((reinterpret_cast<uintptr_t>(bias) | reinterpret_cast<uintptr_t>(Wc)) & 15u) == 0, CAVS_ERR_BAD_ARG,
+               "token_grad_chunks: per-token loss rows need a 16-byte aligned bias and classifier");
   LeafGradArgs lg{mailbox, dOut, dz, Wc, bias, chunk_seg, C, n_leaf, H, ptok, hist, inv_rows, dh_tok, seg_first_chunk};
 #define TOKEN_GRAD(TT, MODE)                                                                                              \
   TokenGradChunks<TT, MODE><<<n_chunks, kThreads, 0, st>>>(partial, static_cast<TT*>(out), chunk_out, static_cast<const TT*>(dA), \

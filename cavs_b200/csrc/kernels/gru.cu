@@ -255,11 +255,6 @@ GruBwdB2(float* __restrict__ mailbox, const float* __restrict__ dHt, const float
   }
 }
 
-// Hidden units per thread: by the width, and by the bias, which starts wherever the parameter blocks before it end.
-int VecWidth(int H, const float* bias = nullptr) {
-  const uintptr_t at = reinterpret_cast<uintptr_t>(bias);
-  return H % 4 == 0 && at % 16 == 0 ? 4 : H % 2 == 0 && at % 8 == 0 ? 2 : 1;
-}
 #define DISPATCH_V(V_, ...)                                   \
   do {                                                        \
     switch (V_) {                                               \

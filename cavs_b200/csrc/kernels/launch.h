@@ -7,6 +7,7 @@
 
 #include <algorithm>
 #include <cstddef>
+#include <cstdint>
 #include <cstdlib>
 
 namespace cavs_b200 {
@@ -47,6 +48,13 @@ inline int GridForElems(size_t n_elems, int threads) {
   const size_t want = (n_elems + threads - 1) / threads;
   const size_t cap = static_cast<size_t>(SmCount()) * ResidentCtas(threads);
   return static_cast<int>(std::max<size_t>(1, std::min(want, cap)));
+}
+
+// Hidden units per thread (4, 2 or 1): by the width, and by where a parameter array that is read at that width starts --
+// the parameter blocks lie one behind the other, so a block starts wherever the ones before it end.
+inline int VecWidth(int H, const float* param = nullptr) {
+  const uintptr_t at = reinterpret_cast<uintptr_t>(param);
+  return H % 4 == 0 && at % 16 == 0 ? 4 : H % 2 == 0 && at % 8 == 0 ? 2 : 1;
 }
 
 // Chained launches (programmatic dependent launch).  A level is a fixed sequence of short kernels, each
