@@ -389,6 +389,8 @@ def run_small_workload(args, name, wl):
     torch.cuda.synchronize()
     ms_e2e = (time.perf_counter() - t0) * 1e3 / args.steps
     clocks = sampler.stop()
+    for eng in engines:
+        eng.read_loss()                          # raises if a bounded wait of any layer's step ran out
     up = engines[0].upload_bytes() if wl["kind"] != "gru" else 0
     n_v = int(scheds[0].n_total)
     line = dict(metric=f"{name}_train_{wl['unit'].split('/')[0]}_per_sec", value=B / (ms_dev * 1e-3), unit=wl["unit"], n_gpus=1, steps=args.steps,

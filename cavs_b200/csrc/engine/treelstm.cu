@@ -49,6 +49,7 @@ struct cavs_treelstm {
   // ---- device workspace views ----
   int32_t* d_idx = nullptr;     // two index blobs of idx_ints each, mirrored by h_idx (pinned)
   int32_t* h_idx = nullptr;
+  int* h_status = nullptr;      // pinned copy of the status word (cavs_treelstm_read), behind h_idx
   size_t idx_ints = 0;
   uint8_t *X = nullptr, *S = nullptr, *HK = nullptr, *dA = nullptr, *ZF = nullptr;   // GEMM operands (fp32 or bf16)
   uint8_t* dAtok = nullptr;     // [distinct tokens, 4H] per-token sums of dA (GEMM operand precision)
@@ -109,6 +110,7 @@ struct cavs_treelstm {
   // the forward cell only forms c and h.  CAVS_GATE_EPILOGUE=0 keeps the separate pre-activation arrays.
   bool gate_epi = false;
   bool narrow = true;          // narrow levels in one persistent launch (CAVS_NARROW_LEVELS=0: level by level)
+  unsigned narrow_polls = kNarrowPolls;   // limit of that launch's waits (CAVS_NARROW_POLLS; 0: every one runs out)
   bool dual_gemm = true;       // small levels: both products of a level in one launch (CAVS_DUAL_GEMM=0: never)
   uint8_t* gates_f = nullptr;
   TcOperandMap map_G3, map_GF;
@@ -301,6 +303,8 @@ void InitModes(cavs_treelstm* e, const cavs_treelstm_config& cfg) {
   e->dual_gemm = !(v3 != nullptr && v3[0] == '0');
   const char* v4 = std::getenv("CAVS_NARROW_LEVELS");
   e->narrow = !(v4 != nullptr && v4[0] == '0');
+  const char* v5 = std::getenv("CAVS_NARROW_POLLS");
+  if (v5 != nullptr) e->narrow_polls = static_cast<unsigned>(std::strtoul(v5, nullptr, 10));
   const char* v2 = std::getenv("CAVS_GATE_EPILOGUE");
   e->gate_epi = e->bf16 && cfg.hidden % 64 == 0 && !(v2 != nullptr && v2[0] == '0');
 }
@@ -499,11 +503,12 @@ extern "C" int cavs_treelstm_create(const cavs_treelstm_config* cfg, void* works
     if (!rc && e->gate_epi) rc = EncodeTcOutput(&e->map_GF, e->gates_f, N * K, H, H, true);
     if (rc) { delete e; return rc; }
   }
-  cudaError_t err = cudaHostAlloc(reinterpret_cast<void**>(&e->h_idx), 2 * e->idx_ints * sizeof(int32_t), cudaHostAllocDefault);
+  cudaError_t err = cudaHostAlloc(reinterpret_cast<void**>(&e->h_idx), (2 * e->idx_ints + 1) * sizeof(int32_t), cudaHostAllocDefault);
   if (err != cudaSuccess) {
     delete e;
     return Fail(CAVS_ERR_CUDA, std::string("treelstm_create: pinned staging: ") + cudaGetErrorString(err));
   }
+  e->h_status = reinterpret_cast<int*>(e->h_idx + 2 * e->idx_ints);
   if (err == cudaSuccess) err = cudaStreamCreateWithFlags(&e->copy_stream, cudaStreamNonBlocking);
   for (int i = 0; i < 2 && err == cudaSuccess; ++i) {
     err = cudaEventCreateWithFlags(&e->copied[i], cudaEventDisableTiming);
@@ -977,7 +982,7 @@ extern "C" int cavs_treelstm_forward(cavs_treelstm* e, void* stream) {
     na.pitch3 = (e->gates_f ? 3 : 3 + K) * H; na.pitch_f = (e->gates_f ? K : 3 + K) * H;
     na.A = e->A; na.a_row = bt.tok_slot; na.bias = B; na.U_iou = U_iou; na.U_f = U_f;
     na.child = e->leaf_tok ? bt.child_st : bt.child; na.level_off = bt.lev;
-    na.barrier = e->barriers + i; na.status = e->Status();
+    na.barrier = e->barriers + i; na.status = e->Status(); na.polls = e->narrow_polls;
     na.n_total = nt; na.level_begin = narrow[i].begin; na.level_end = narrow[i].end; na.H = H;
     const double rows = bt.level_off[narrow[i].end] - bt.level_off[narrow[i].begin];
     PROF(e, kProfGemm, 2.0 * rows * H * H * (3 + K), st, e->bf16 ? LaunchNarrowForwardBf16(narrow[i].plan, na, K, st) : LaunchNarrowForwardF32(narrow[i].plan, na, K, st));
@@ -1076,7 +1081,7 @@ extern "C" int cavs_treelstm_backward(cavs_treelstm* e, void* stream) {
     na.gates_f = e->gates_f ? e->gates_f : e->gates + static_cast<size_t>(3) * H * e->elt;
     na.pitch3 = (e->gates_f ? 3 : 3 + K) * H; na.pitch_f = (e->gates_f ? K : 3 + K) * H;
     na.child = bt.child; na.child_state = e->leaf_tok ? bt.child_st : nullptr; na.parent = bt.parent; na.level_off = bt.lev;
-    na.barrier = e->barriers + 2 + i; na.status = e->Status();
+    na.barrier = e->barriers + 2 + i; na.status = e->Status(); na.polls = e->narrow_polls;
     na.n_total = nt; na.level_begin = narrow[i].begin; na.level_end = narrow[i].end; na.H = H;
     const double rows = bt.level_off[narrow[i].end] - bt.level_off[narrow[i].begin];
     PROF(e, kProfGemm, 2.0 * rows * H * H * (3 + K), st, e->bf16 ? LaunchNarrowBackwardBf16(narrow[i].plan, na, K, st) : LaunchNarrowBackwardF32(narrow[i].plan, na, K, st));
@@ -1438,6 +1443,22 @@ extern "C" int cavs_treelstm_read_loss(cavs_treelstm* e, float* loss_sum_host, i
   std::memcpy(&status, &host[1], sizeof(int));
   if (status_host) *status_host = status;
   CAVS_REQUIRE(status == 0, CAVS_ERR_TIMEOUT, "treelstm: a bounded device-side wait expired during the step");
+  return CAVS_OK;
+}
+
+extern "C" int cavs_treelstm_read(cavs_treelstm* e, int what, void* host, size_t bytes, void* stream) {
+  CAVS_REQUIRE(e && (host || bytes == 0), CAVS_ERR_BAD_ARG, "treelstm_read: null pointer");
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  if (bytes > 0) {
+    const void* dev = nullptr;
+    size_t have = 0;
+    if (int rc = cavs_treelstm_peek(e, what, &dev, &have)) return rc;
+    CAVS_REQUIRE(bytes <= have, CAVS_ERR_BAD_ARG, "treelstm_read: the array has " + std::to_string(have) + " bytes");
+    CAVS_CUDA(cudaMemcpyAsync(host, dev, bytes, cudaMemcpyDeviceToHost, st));
+  }
+  CAVS_CUDA(cudaMemcpyAsync(e->h_status, e->Status(), sizeof(int), cudaMemcpyDeviceToHost, st));
+  CAVS_CUDA(cudaStreamSynchronize(st));
+  CAVS_REQUIRE(*e->h_status == 0, CAVS_ERR_TIMEOUT, "treelstm: a bounded device-side wait expired");
   return CAVS_OK;
 }
 

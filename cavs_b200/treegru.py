@@ -82,6 +82,7 @@ class TreeGRU:
         off = p.value - self.workspace.data_ptr()
         t = self.workspace[off:off + nbytes.value].view(torch.float32)
         torch.cuda.synchronize()
+        self.read_loss()                     # raises if a bounded device-side wait ran out
         return t.cpu().numpy().reshape(shape)
 
     def state(self) -> np.ndarray:
@@ -92,5 +93,6 @@ class TreeGRU:
 
     def grad_dict(self) -> dict:
         torch.cuda.synchronize()
+        self.read_loss()
         g = self.grads.cpu().numpy()
         return {"d" + k: g[self.offsets[k]:self.offsets[k] + self.sizes[k]].copy() for k in self.PARAM_NAMES}

@@ -189,14 +189,19 @@ class TreeLSTM:
                                  ctypes.c_float(lr), ctypes.c_float(eps), _stream()))
         self.refresh_weights()
 
+    def check_waits(self) -> None:
+        """Raises if a bounded device-side wait of any pass so far ran out; synchronises the current stream.  read_loss(),
+        state(), loss_rows(), peek() and grad_dict() check by themselves: this is for callers of device_view() alone."""
+        check(lib().cavs_treelstm_read(self._h, 0, None, ctypes.c_size_t(0), _stream()))
+
     def peek(self, what: int, shape) -> np.ndarray:
         p = ctypes.c_void_p()
         nbytes = ctypes.c_size_t()
         check(lib().cavs_treelstm_peek(self._h, what, ctypes.byref(p), ctypes.byref(nbytes)))
-        off = p.value - self.workspace.data_ptr()
-        t = self.workspace[off:off + nbytes.value].view(torch.float32)
+        out = np.empty(nbytes.value // 4, np.float32)
         torch.cuda.synchronize()
-        return t.cpu().numpy().reshape(shape)
+        check(lib().cavs_treelstm_read(self._h, what, ptr(out), nbytes, _stream()))
+        return out.reshape(shape)
 
     def state(self) -> np.ndarray:
         check(lib().cavs_treelstm_materialize_state(self._h, _stream()))   # leaf rows may live per token
@@ -208,5 +213,6 @@ class TreeLSTM:
 
     def grad_dict(self) -> dict:
         torch.cuda.synchronize()
+        self.check_waits()
         g = self.grads.cpu().numpy()
         return {"d" + k: g[self.offsets[k]:self.offsets[k] + self.sizes[k]].copy() for k in self.PARAM_NAMES}

@@ -415,6 +415,10 @@ CAVS_API int cavs_treelstm_profile_read(cavs_treelstm* e, double* ms, double* wo
  * 6 the two words cavs_treelstm_read_loss copies: loss sum (float) and status (int) -- for callers that fetch
  * them with their own asynchronous copy instead of the blocking read. */
 CAVS_API int cavs_treelstm_peek(cavs_treelstm* e, int what, const void** dev_ptr, size_t* bytes);
+/* The first `bytes` bytes of peek array `what`, copied to host memory behind the work enqueued on `stream`; synchronises it.
+ * CAVS_ERR_TIMEOUT when a bounded device-side wait of any pass so far expired (the word stays raised), so that a caller
+ * that reads no loss -- a forward pass, a layer without a loss head -- sees it too.  bytes == 0: that check alone. */
+CAVS_API int cavs_treelstm_read(cavs_treelstm* e, int what, void* host, size_t bytes, void* stream);
 
 /* ------------------------------------------------------------------------ */
 /* Child-sum Tree-GRU engine: the same level loop over a second vertex        */
