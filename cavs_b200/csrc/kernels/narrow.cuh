@@ -81,25 +81,23 @@ struct BulkRows {
     __syncwarp();
     if (src != nullptr) bulk::Load(dst + lane * pitch, src, bytes, bar);
   }
-  __device__ __forceinline__ bool Poll(int buf, unsigned polls) const {
-    const uint32_t bar = bulk::SmemAddr(bars + buf), parity = (phases >> buf) & 1;
-    for (unsigned it = 0; it < polls; ++it) {
-      uint32_t done;
-      asm volatile(
-          "{\n\t.reg .pred p;\n\t"
-          "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, 1000;\n\t"
-          "selp.u32 %0, 1, 0, p;\n\t}"
-          : "=r"(done) : "r"(bar), "r"(parity) : "memory");
-      if (done) return true;
-    }
-    return false;
-  }
-  // By all threads.  An expired wait raises *status and waits once more: the copies are under way into this CTA's memory,
-  // which must not be given back before they land.  After that nothing is waited for any more.
+  // By all threads.  A wait that expires raises *status and goes on to twice the ordinary limit: the copies are under way
+  // into this CTA's memory, which must not be given back before they land.  After that nothing is waited for any more.
   __device__ __forceinline__ void Wait(int buf, unsigned polls, int* status) {
-    if (ok && !Poll(buf, polls)) {
-      atomicExch(status, 1);
-      ok = Poll(buf, kNarrowPolls);
+    if (ok) {
+      const uint32_t bar = bulk::SmemAddr(bars + buf), parity = (phases >> buf) & 1;
+      ok = false;
+      for (unsigned it = 0; it < 2 * kNarrowPolls && !ok; ++it) {
+        if (it == polls) atomicExch(status, 1);
+        uint32_t done;
+        asm volatile(
+            "{\n\t.reg .pred p;\n\t"
+            "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, 1000;\n\t"
+            "selp.u32 %0, 1, 0, p;\n\t}"
+            : "=r"(done) : "r"(bar), "r"(parity) : "memory");
+        ok = done != 0;
+      }
+      if (!ok) atomicExch(status, 1);
     }
     phases ^= 1u << buf;
   }
