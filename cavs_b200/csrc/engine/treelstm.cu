@@ -110,7 +110,7 @@ struct cavs_treelstm {
   // the forward cell only forms c and h.  CAVS_GATE_EPILOGUE=0 keeps the separate pre-activation arrays.
   bool gate_epi = false;
   bool narrow = true;          // narrow levels in one persistent launch (CAVS_NARROW_LEVELS=0: level by level)
-  unsigned narrow_polls = kNarrowPolls;   // limit of that launch's waits (CAVS_NARROW_POLLS; 0: every one runs out)
+  unsigned narrow_withhold = 0;   // CAVS_NARROW_WITHHOLD=1: its grid barrier never completes, so that the wait runs out
   bool dual_gemm = true;       // small levels: both products of a level in one launch (CAVS_DUAL_GEMM=0: never)
   uint8_t* gates_f = nullptr;
   TcOperandMap map_G3, map_GF;
@@ -303,8 +303,8 @@ void InitModes(cavs_treelstm* e, const cavs_treelstm_config& cfg) {
   e->dual_gemm = !(v3 != nullptr && v3[0] == '0');
   const char* v4 = std::getenv("CAVS_NARROW_LEVELS");
   e->narrow = !(v4 != nullptr && v4[0] == '0');
-  const char* v5 = std::getenv("CAVS_NARROW_POLLS");
-  if (v5 != nullptr) e->narrow_polls = static_cast<unsigned>(std::strtoul(v5, nullptr, 10));
+  const char* v5 = std::getenv("CAVS_NARROW_WITHHOLD");
+  e->narrow_withhold = v5 != nullptr && v5[0] == '1';
   const char* v2 = std::getenv("CAVS_GATE_EPILOGUE");
   e->gate_epi = e->bf16 && cfg.hidden % 64 == 0 && !(v2 != nullptr && v2[0] == '0');
 }
@@ -982,7 +982,7 @@ extern "C" int cavs_treelstm_forward(cavs_treelstm* e, void* stream) {
     na.pitch3 = (e->gates_f ? 3 : 3 + K) * H; na.pitch_f = (e->gates_f ? K : 3 + K) * H;
     na.A = e->A; na.a_row = bt.tok_slot; na.bias = B; na.U_iou = U_iou; na.U_f = U_f;
     na.child = e->leaf_tok ? bt.child_st : bt.child; na.level_off = bt.lev;
-    na.barrier = e->barriers + i; na.status = e->Status(); na.polls = e->narrow_polls;
+    na.barrier = e->barriers + i; na.status = e->Status(); na.withhold = e->narrow_withhold;
     na.n_total = nt; na.level_begin = narrow[i].begin; na.level_end = narrow[i].end; na.H = H;
     const double rows = bt.level_off[narrow[i].end] - bt.level_off[narrow[i].begin];
     PROF(e, kProfGemm, 2.0 * rows * H * H * (3 + K), st, e->bf16 ? LaunchNarrowForwardBf16(narrow[i].plan, na, K, st) : LaunchNarrowForwardF32(narrow[i].plan, na, K, st));
@@ -1081,7 +1081,7 @@ extern "C" int cavs_treelstm_backward(cavs_treelstm* e, void* stream) {
     na.gates_f = e->gates_f ? e->gates_f : e->gates + static_cast<size_t>(3) * H * e->elt;
     na.pitch3 = (e->gates_f ? 3 : 3 + K) * H; na.pitch_f = (e->gates_f ? K : 3 + K) * H;
     na.child = bt.child; na.child_state = e->leaf_tok ? bt.child_st : nullptr; na.parent = bt.parent; na.level_off = bt.lev;
-    na.barrier = e->barriers + 2 + i; na.status = e->Status(); na.polls = e->narrow_polls;
+    na.barrier = e->barriers + 2 + i; na.status = e->Status(); na.withhold = e->narrow_withhold;
     na.n_total = nt; na.level_begin = narrow[i].begin; na.level_end = narrow[i].end; na.H = H;
     const double rows = bt.level_off[narrow[i].end] - bt.level_off[narrow[i].begin];
     PROF(e, kProfGemm, 2.0 * rows * H * H * (3 + K), st, e->bf16 ? LaunchNarrowBackwardBf16(narrow[i].plan, na, K, st) : LaunchNarrowBackwardF32(narrow[i].plan, na, K, st));

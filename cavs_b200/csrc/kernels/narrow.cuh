@@ -19,6 +19,7 @@ namespace narrow {
 
 constexpr int kThreads = 512, kWarps = kThreads / 32;
 constexpr size_t kMaxSmem = 226 * 1024;
+constexpr unsigned kBarrierPolls = 1u << 19;   // about half a second
 
 // The cell kernels' activations (kernels/cell.cu): libm-accurate for fp32, exp2-unit forms for bf16.
 template <bool kFast>
@@ -39,11 +40,11 @@ __device__ __forceinline__ void GridArrive(unsigned* counter) {
   __syncthreads();
   if (threadIdx.x == 0) asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(counter) : "memory");
 }
-__device__ __forceinline__ bool GridWait(unsigned* counter, unsigned target, unsigned polls, int* status) {
+__device__ __forceinline__ bool GridWait(unsigned* counter, unsigned target, int* status) {
   __shared__ int s_ok;
   if (threadIdx.x == kThreads - 32) {   // a warp with few or no rows of its own to request
     int ok = 0;
-    for (unsigned it = 0; it < polls; ++it) {
+    for (unsigned it = 0; it < kBarrierPolls; ++it) {
       unsigned v;
       asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(counter) : "memory");
       if (v >= target) { ok = 1; break; }
@@ -81,14 +82,12 @@ struct BulkRows {
     __syncwarp();
     if (src != nullptr) bulk::Load(dst + lane * pitch, src, bytes, bar);
   }
-  // By all threads.  A wait that expires raises *status and goes on to twice the ordinary limit: the copies are under way
-  // into this CTA's memory, which must not be given back before they land.  After that nothing is waited for any more.
-  __device__ __forceinline__ void Wait(int buf, unsigned polls, int* status) {
+  // By all threads; after one expired wait nothing is waited for any more (and *status is raised) before Drain.
+  __device__ __forceinline__ void Wait(int buf, int* status) {
     if (ok) {
       const uint32_t bar = bulk::SmemAddr(bars + buf), parity = (phases >> buf) & 1;
       ok = false;
-      for (unsigned it = 0; it < 2 * kNarrowPolls && !ok; ++it) {
-        if (it == polls) atomicExch(status, 1);
+      for (uint32_t it = 0; it < (1u << 18) && !ok; ++it) {
         uint32_t done;
         asm volatile(
             "{\n\t.reg .pred p;\n\t"
@@ -100,6 +99,20 @@ struct BulkRows {
       if (!ok) atomicExch(status, 1);
     }
     phases ^= 1u << buf;
+  }
+  // Before the CTA ends: after an expired wait, copies may still be under way into its memory.  Bounded as well.
+  __device__ __forceinline__ void Drain() const {
+    if (ok) return;
+    for (int buf = 0; buf < kBuffers; ++buf)
+      for (uint32_t it = 0; it < (1u << 18); ++it) {
+        uint32_t done;
+        asm volatile(
+            "{\n\t.reg .pred p;\n\t"
+            "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, 1000;\n\t"
+            "selp.u32 %0, 1, 0, p;\n\t}"
+            : "=r"(done) : "r"(bulk::SmemAddr(bars + buf)), "r"(((phases >> buf) & 1) ^ 1) : "memory");   // the last phase waited for
+        if (done) break;
+      }
   }
 };
 

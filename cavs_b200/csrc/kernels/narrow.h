@@ -22,8 +22,8 @@ NarrowPlan PlanNarrowBf16(int H, int K, int rows, bool backward);
 // Levels [level_begin, level_end) in ascending order; level_off: device copy of the level offsets.  Arrays as for the
 // per-level launches (kernels/cell.h): S / HK, the saved gates and h|c of every row are written.  A, S, HK and the
 // weights are fp32, or bf16 with fp16 gates; i|o|u of row t at gates + t * pitch3, f_0.. at gates_f + t * pitch_f.
-// barrier: a zeroed word; status: raised when a bounded wait expires; polls: its limit.
-constexpr unsigned kNarrowPolls = 1u << 19;   // about half a second
+// barrier: a zeroed word; status: raised when a bounded wait expires; withhold: 1 keeps the
+// grid barrier from ever completing (a test of its wait).
 struct NarrowForwardArgs {
   float* state;
   void *gates, *gates_f, *S, *HK;
@@ -32,7 +32,7 @@ struct NarrowForwardArgs {
   const int32_t *child, *a_row, *level_off;   // child: state rows of the children
   unsigned* barrier;
   int* status;
-  unsigned polls;
+  unsigned withhold;
   long long pitch3, pitch_f;
   int n_total, level_begin, level_end, H;
   int w, col_groups, row_groups, buffers;     // from the plan
@@ -50,7 +50,7 @@ struct NarrowBackwardArgs {
   const int32_t *child, *child_state, *parent, *level_off;
   unsigned* barrier;
   int* status;
-  unsigned polls;
+  unsigned withhold;
   long long pitch3, pitch_f;
   int n_total, level_begin, level_end, H, C;
   int w, col_groups, row_groups, buffers;     // from the plan

@@ -197,7 +197,7 @@ __global__ void __launch_bounds__(kThreads, 1) NarrowForwardBf16(const NarrowFor
     if (l + 1 < a.level_end) {
       GridArrive(a.barrier);
       prefetch(off, end, rg);
-      if (!GridWait(a.barrier, ++barrier * gridDim.x, a.polls, a.status)) return;
+      if (!GridWait(a.barrier, ++barrier * gridDim.x + a.withhold, a.status)) break;
     }
   }
 }
@@ -239,7 +239,7 @@ __global__ void __launch_bounds__(kThreads, 1) NarrowBackwardBf16(const NarrowBa
     gg.Level(a, off, end);
     GridArrive(a.barrier);
     if (l > a.level_begin) gg.Request(a, next_off, off);   // only the mailbox rows are not complete yet
-    if (!GridWait(a.barrier, ++barrier * gridDim.x, a.polls, a.status)) return;
+    if (!GridWait(a.barrier, ++barrier * gridDim.x + a.withhold, a.status)) break;
     const int tiles = (end - off + TR - 1) / TR;
     for (int tile = rg; tile < tiles; tile += a.row_groups) {
       const int t0 = off + tile * TR, rows = min(TR, end - t0);
@@ -269,7 +269,7 @@ __global__ void __launch_bounds__(kThreads, 1) NarrowBackwardBf16(const NarrowBa
       for (int q = 0; q < ahead; ++q) load(q);
 #pragma unroll
       for (int q = 0; q < G; ++q) {
-        ring.Wait(q % a.buffers, a.polls, a.status);
+        ring.Wait(q % a.buffers, a.status);
         for (int st = step_begin; st < step_end; ++st) {
           uint32_t b[2];
           LdMatrix2(b, b_addr + min(q, 3) * kUnits * pk * 2 + st * 32);
@@ -315,10 +315,11 @@ __global__ void __launch_bounds__(kThreads, 1) NarrowBackwardBf16(const NarrowBa
       __syncthreads();   // the next level's rows of these columns were written by this CTA
     } else if (l > a.level_begin) {
       GridArrive(a.barrier);
-      if (!GridWait(a.barrier, ++barrier * gridDim.x, a.polls, a.status)) return;
+      if (!GridWait(a.barrier, ++barrier * gridDim.x + a.withhold, a.status)) break;
     }
   }
   gg.FoldSums(a, red);
+  ring.Drain();
 }
 
 }  // namespace

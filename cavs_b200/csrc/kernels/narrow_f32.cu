@@ -209,7 +209,7 @@ __global__ void __launch_bounds__(kThreads, 1) NarrowForward(const NarrowForward
         prefetch(off, end, tile + a.row_groups);
         if (a.buffers == 2 && threadIdx.x < K * TR) s_child[buf ^ 1][threadIdx.x / TR][threadIdx.x % TR] = child;
       }
-      if constexpr (V == 4) ring.Wait(nbuf, a.polls, a.status);
+      if constexpr (V == 4) ring.Wait(nbuf, a.status);
       __syncthreads();
       if (more && a.buffers == 2) load_rows(tile + a.row_groups, buf ^ 1);   // arrives under this tile's products
       const float* At = At0 + nbuf * K * TR * p;
@@ -253,9 +253,10 @@ __global__ void __launch_bounds__(kThreads, 1) NarrowForward(const NarrowForward
     if (l + 1 < a.level_end) {
       GridArrive(a.barrier);
       prefetch(off, end, rg);
-      if (!GridWait(a.barrier, ++barrier * gridDim.x, a.polls, a.status)) return;
+      if (!GridWait(a.barrier, ++barrier * gridDim.x + a.withhold, a.status)) break;
     }
   }
+  ring.Drain();
 }
 
 // ---- backward ----
@@ -321,7 +322,7 @@ __device__ __forceinline__ void BwdTile(const NarrowBackwardArgs& a, const float
   for (int q = 0; q < ahead; ++q) load(q);
 #pragma unroll
   for (int q = 0; q < G; ++q) {
-    if constexpr (V == 4) ring.Wait(q % a.buffers, a.polls, a.status);
+    if constexpr (V == 4) ring.Wait(q % a.buffers, a.status);
     else __syncthreads();
     const float* buf = At + (q % a.buffers) * TR * p;
     const float* wt = Wt + unit * pw + min(q, 3) * hk;
@@ -391,7 +392,7 @@ __global__ void __launch_bounds__(kThreads, 1) NarrowBackward(const NarrowBackwa
     gg.Level(a, off, end);
     GridArrive(a.barrier);
     if (l > a.level_begin) gg.Request(a, next_off, off);   // only the mailbox rows are not complete yet
-    if (!GridWait(a.barrier, ++barrier * gridDim.x, a.polls, a.status)) return;
+    if (!GridWait(a.barrier, ++barrier * gridDim.x + a.withhold, a.status)) break;
     const int tiles = (end - off + TR - 1) / TR;
     for (int tile = rg; tile < tiles; tile += a.row_groups) {
       const int t0 = off + tile * TR, rows = min(TR, end - t0);
@@ -403,10 +404,11 @@ __global__ void __launch_bounds__(kThreads, 1) NarrowBackward(const NarrowBackwa
       __syncthreads();   // the next level's rows of these columns were written by this CTA
     } else if (l > a.level_begin) {
       GridArrive(a.barrier);
-      if (!GridWait(a.barrier, ++barrier * gridDim.x, a.polls, a.status)) return;
+      if (!GridWait(a.barrier, ++barrier * gridDim.x + a.withhold, a.status)) break;
     }
   }
   gg.FoldSums(a, red);
+  ring.Drain();
 }
 
 size_t ForwardSmem(int H, int K, int w, int buffers) {

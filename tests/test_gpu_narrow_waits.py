@@ -1,6 +1,6 @@
-"""The bounded waits of the narrow levels' persistent launches, and two engines that use the GPU at once.  With a poll limit
-of zero every wait runs out: the launches raise the engine's status word and return with levels unwritten, whoever takes
-results to the host gets CAVS_ERR_TIMEOUT, and the context stays usable."""
+"""The bounded waits of the narrow levels' persistent launches, and two engines that use the GPU at once.  With a grid
+barrier that never completes its wait runs out (half a second): the launches raise the engine's status word and return with
+levels unwritten, whoever takes results to the host gets CAVS_ERR_TIMEOUT, and the context stays usable."""
 import threading
 
 import numpy as np
@@ -38,7 +38,7 @@ def test_expired_waits_reach_the_caller(cuda, monkeypatch, bf16, H, K, C):
     label = label % max(C, 1)
     params = make_params(2, H, E, V, max(C, 1))
     args = (H, E, V, C, K, bf16, parents, tok, label if C else None, params)
-    monkeypatch.setenv("CAVS_NARROW_POLLS", "0")
+    monkeypatch.setenv("CAVS_NARROW_WITHHOLD", "1")
     eng = _engine(*args)
     eng.forward()
     for call in (eng.state, eng.check_waits, eng.grad_dict):
@@ -49,8 +49,8 @@ def test_expired_waits_reach_the_caller(cuda, monkeypatch, bf16, H, K, C):
     eng.backward()
     for call in (eng.read_loss, eng.loss_rows, eng.grad_dict):
         _times_out(call)
-    # the same step in the same process with the ordinary limit
-    monkeypatch.delenv("CAVS_NARROW_POLLS")
+    # the same step in the same process without it
+    monkeypatch.delenv("CAVS_NARROW_WITHHOLD")
     good = _engine(*args)
     good.forward()
     if C == 0:
