@@ -404,53 +404,69 @@ int Gemm(cavs_treelstm* e, void* c, long long ldc, int accumulate, const void* a
   return CAVS_OK;
 }
 
+// Microseconds of one fp32 level launched kernel by kernel, inside a chain of such levels (fitted to the same levels as
+// NarrowLevelUsF32: root mean square error 8 % forward, 9 % backward).
+double PerLevelUsF32(const cavs_treelstm* e, int rows, bool backward) {
+  const int H = e->cfg.hidden, K = e->cfg.n_slots;
+  const double elems = 1e-6 * rows * H * (K + 2), runs = H % 4 == 0 ? 0.0 : 1e-6 * rows * H * (3 + K);   // runs: rows of no whole 16-byte words
+  const double products = backward ? GemmF32Us(rows, H, 3 * H, e->splitk_bytes) + GemmF32Us(rows * K, H, H, e->splitk_bytes)
+                                   : GemmF32Us(rows, 3 * H, H, e->splitk_bytes) + GemmF32Us(rows * K, H, H, e->splitk_bytes);
+  return backward ? 1.41 * products + 5.8 * elems + 1.03e-3 * rows * (K + 2) + 24.4 * runs : 4.6 + products + 4.2 * elems + 3.6 * runs;
+}
+
 // Narrow levels run as one persistent launch (kernels/narrow_f32.cu, narrow_bf16.cu).  The level sizes of a schedule do
 // not increase, so they are a suffix of the levels: from the first one that the persistent kernel is estimated to finish
-// sooner than the per-level launches.
-// fp32: a per-level level costs 25 us forward and 31 backward up to some hundred rows; the persistent one 4 and 9 us and
-// 1 us per 7e6 (forward) or 3.3e6 (backward) multiply-adds (H = 512, one child slot): the line lies below where they meet.
-// bf16: per level 16 us forward and 23 us backward at H = 512, 18 and 30 at 1024 (launch and fill floors).
+// clearly sooner than the per-level launches.  A launch costs 7 to 12 us beside its levels (its weights' way into shared
+// memory).  Us saved per level, seen in chains of levels of one size with a loss head of five classes, forward / backward:
+//   fp32  H = 512, one slot    16.7 / 12.5 at 64 rows, 12.7 / 0.6 at 128, 4.2 / -18 at 256
+//         H = 150, two slots   19.0 / 17.6 at 128, 12.5 / 8.9 at 256, 8.4 / -2.2 at 512
+//         H = 32, two slots    7.8 / 10.8 at 2048, 2.5 / 2.9 at 4096, -9.0 / -9.9 at 8192
+//   bf16  H = 1024, two slots  5.7 / 12.1 at 16, 1.4 / 4.9 at 32, -6.5 / -7.4 at 64
+//         H = 512, one slot    5.3 / 4.7 at 64, 2.0 / 4.8 at 128, -4.0 / -4.0 at 256
+// fp32: by estimates of both; the margins keep out levels that the estimates' errors would make slower (over 300 sizes they
+// give away 100 of 5280 us; one product of rows and widths for all sizes gave away 290, up to 29 us in one level).
+// bf16: per level 11 us forward and 21 backward at H = 1024 (10 and 17 at 512), more without the fused loss head's streaming
+// cell; the plan's estimate and the line it is held against are both about 1.4 times that, and the line lies where the signs
+// above change (over 200 sizes it gives away 23 of the 2068 us that could be saved).
 struct NarrowRange { int begin, end; NarrowPlan plan; };
 std::vector<NarrowRange> NarrowLevels(const cavs_treelstm* e, const cavs_treelstm::Batch& bt, bool backward) {
   std::vector<NarrowRange> out;
-  const int H = e->cfg.hidden, K = e->cfg.n_slots;
-  auto rows = [&](int l) { return bt.level_off[l + 1] - bt.level_off[l]; };
-  int begin = bt.l1 ? 2 : 1;
   if (!e->narrow) return out;
-  if (e->bf16) {
-    const double per_level = backward ? 16.0 + H / 75.0 : 13.0 + H / 200.0;
-    while (begin < bt.n_levels && rows(begin) > 0 && PlanNarrowBf16(H, K, rows(begin), backward).level_us > 0.8 * per_level) ++begin;
-    if (begin >= bt.n_levels) return out;
-    // Two launches where the levels of one row tile are many: those run backward with one row group, one barrier a level.
-    int split = begin;
-    while (split < bt.n_levels && rows(split) > (K == 1 ? 32 : 16)) ++split;
-    const NarrowPlan wide = PlanNarrowBf16(H, K, rows(begin), backward);
-    if (wide.w == 0) return out;
-    if (split > begin && bt.n_levels - split >= 6 && wide.row_groups > 1) {
-      out.push_back({begin, split, wide});
-      out.push_back({split, bt.n_levels, PlanNarrowBf16(H, K, rows(split), backward)});
-    } else {
-      out.push_back({begin, bt.n_levels, wide});
-    }
-    return out;
+  const int H = e->cfg.hidden, K = e->cfg.n_slots, n = bt.n_levels;
+  const double bf16_line = 0.8 * (backward ? 16.0 + H / 75.0 : 13.0 + H / 200.0), f32_margin = backward ? 0.85 : 0.9;
+  auto rows = [&](int l) { return bt.level_off[l + 1] - bt.level_off[l]; };
+  auto plan = [&](int r) { return e->bf16 ? PlanNarrowBf16(H, K, r, backward) : PlanNarrowF32(H, K, r, backward); };
+  NarrowPlan wide;
+  int begin = bt.l1 ? 2 : 1;
+  for (int seen = 0; begin < n; ++begin) {
+    if (rows(begin) == seen) continue;
+    seen = rows(begin);
+    if (seen <= 0) return out;
+    wide = plan(seen);
+    if (wide.w == 0) return out;   // slices and rows do not fit: fp32 H above 576 (two slots) to 768 (one) forward, 704 to 1024
+                                   // backward; bf16 1184, forward 1152, 896 and 768 with two, three and four slots
+    if (e->bf16 ? wide.level_us <= bf16_line : NarrowLevelUsF32(wide, H, K, seen, backward) < f32_margin * PerLevelUsF32(e, seen, backward)) break;
   }
-  while (begin < bt.n_levels && static_cast<double>(rows(begin)) * H * H * (3 + K) > (backward ? 6e7 : 1.2e8)) ++begin;
-  if (begin >= bt.n_levels) return out;
-  // Two launches when the upper levels are much narrower: few rows want few hidden units per CTA, so that all CTAs
-  // take part; many rows want many, so that a gathered row is used more often.
+  if (begin >= n || (e->bf16 && begin == n - 1)) return out;   // (a single bf16 level saves less than its launch costs)
+  // Two launches where the upper levels are much narrower.  fp32: few rows want few hidden units per CTA, so that all CTAs
+  // take part; many rows want many, so that a gathered row is used more often.  bf16: levels of one row tile run backward
+  // with one row group, one barrier a level.
   int split = begin;
-  while (split < bt.n_levels && rows(split) > 96) ++split;
-  const NarrowPlan wide = PlanNarrowF32(H, K, rows(begin), backward);
-  if (wide.w == 0) return out;
-  if (split > begin && bt.n_levels - split >= 4) {
-    const NarrowPlan low = PlanNarrowF32(H, K, rows(split), backward);
-    if (low.w != wide.w && low.w != 0) {
-      out.push_back({begin, split, wide});
-      out.push_back({split, bt.n_levels, low});
-      return out;
+  while (split < n && rows(split) > (e->bf16 ? (K == 1 ? 32 : 16) : 96)) ++split;
+  out.push_back({begin, n, wide});
+  if (split > begin && n - split >= (e->bf16 ? 6 : 4)) {
+    const NarrowPlan low = plan(rows(split));
+    if (e->bf16 ? wide.row_groups > 1 : low.w != wide.w && low.w != 0) {
+      out[0].end = split;
+      out.push_back({split, n, low});
     }
   }
-  out.push_back({begin, bt.n_levels, wide});
+  if (!e->bf16) {   // the launches have to pay (the narrower a level the more it saves: the rest is gain then)
+    double gain = -9.0 * out.size();
+    for (const NarrowRange& r : out)
+      for (int l = r.begin; l < r.end && gain <= 0.0; ++l) gain += PerLevelUsF32(e, rows(l), backward) - NarrowLevelUsF32(r.plan, H, K, rows(l), backward);
+    if (gain <= 0.0) out.clear();
+  }
   return out;
 }
 
@@ -1449,14 +1465,15 @@ extern "C" int cavs_treelstm_read_loss(cavs_treelstm* e, float* loss_sum_host, i
 extern "C" int cavs_treelstm_read(cavs_treelstm* e, int what, void* host, size_t bytes, void* stream) {
   CAVS_REQUIRE(e && (host || bytes == 0), CAVS_ERR_BAD_ARG, "treelstm_read: null pointer");
   cudaStream_t st = static_cast<cudaStream_t>(stream);
+  const void* dev = nullptr;
+  size_t have = 0;
   if (bytes > 0) {
-    const void* dev = nullptr;
-    size_t have = 0;
     if (int rc = cavs_treelstm_peek(e, what, &dev, &have)) return rc;
     CAVS_REQUIRE(bytes <= have, CAVS_ERR_BAD_ARG, "treelstm_read: the array has " + std::to_string(have) + " bytes");
-    CAVS_CUDA(cudaMemcpyAsync(host, dev, bytes, cudaMemcpyDeviceToHost, st));
   }
+  // (into pinned memory and first, so that it is under way while the copy into the caller's pageable memory is set up)
   CAVS_CUDA(cudaMemcpyAsync(e->h_status, e->Status(), sizeof(int), cudaMemcpyDeviceToHost, st));
+  if (bytes > 0) CAVS_CUDA(cudaMemcpyAsync(host, dev, bytes, cudaMemcpyDeviceToHost, st));
   CAVS_CUDA(cudaStreamSynchronize(st));
   CAVS_REQUIRE(*e->h_status == 0, CAVS_ERR_TIMEOUT, "treelstm: a bounded device-side wait expired");
   return CAVS_OK;

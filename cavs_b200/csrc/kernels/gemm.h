@@ -122,6 +122,8 @@ struct GemmF32Args {
   int k_per_split = 0;   // set by GemmF32 (0: no split)
 };
 int GemmF32(const GemmF32Args& args, cudaStream_t stream);
+// Estimated microseconds of a product with `scratch_bytes` of scratch (the estimate by which GemmF32 chooses its kernel).
+double GemmF32Us(int m, int n, int k, size_t scratch_bytes);
 // The tensor-core kernel alone: tiles of 128 x tile_n (128 or 64).  k is cut over *splits CTAs per tile (rewritten with
 // the number used); with more than one the partial products are left in args.scratch [splits, m, n].
 int GemmF32Split(const GemmF32Args& args, int tile_n, int* splits, cudaStream_t stream);

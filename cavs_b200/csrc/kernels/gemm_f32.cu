@@ -115,9 +115,9 @@ __global__ void __launch_bounds__(256) GemmF32Reduce(float* __restrict__ c, long
 
 // k splits of the FFMA kernel: few tiles and a long k loop go to enough CTAs to fill the machine once (at least 64 k
 // per split).
-int PlainSplits(const GemmF32Args& g, long long tiles) {
-  if (g.scratch == nullptr || tiles >= SmCount() || g.k < 256) return 1;
-  int splits = static_cast<int>(std::min<long long>(std::min<long long>(16, g.k / 64), (2LL * SmCount()) / tiles));
+int PlainSplits(const GemmF32Args& g, long long tiles, int sms) {
+  if (g.scratch_bytes == 0 || tiles >= sms || g.k < 256) return 1;
+  int splits = static_cast<int>(std::min<long long>(std::min<long long>(16, g.k / 64), (2LL * sms) / tiles));
   while (splits > 1 && static_cast<size_t>(splits) * g.m * g.n * sizeof(float) > g.scratch_bytes) --splits;
   return splits;
 }
@@ -128,18 +128,43 @@ double ReduceCost(const GemmF32Args& g, int splits) {
   return splits > 1 ? 2.0 + 4.0 * (splits + 1) * g.m * g.n / 3e6 : 0.0;
 }
 // FFMA: a 16-wide k step costs 0.92 us of latency, or 0.77 us of arithmetic for each CTA that shares the SM.
-double PlainCost(const GemmF32Args& g, long long tiles, int splits) {
+double PlainCost(const GemmF32Args& g, long long tiles, int splits, int sms) {
   const double steps = ((g.k + splits - 1) / splits + kTK - 1) / kTK;
-  return 3.5 + steps * std::max(0.92, 0.77 * ((tiles * splits + SmCount() - 1) / SmCount())) + ReduceCost(g, splits);
+  return 3.5 + steps * std::max(0.92, 0.77 * ((tiles * splits + sms - 1) / sms)) + ReduceCost(g, splits);
 }
 // Tensor cores: a 64-wide k block costs 2.2 us with 128 columns per tile, 1.95 us with 64.
-double SplitCost(const GemmF32Args& g, int tile_n, int splits) {
+double SplitCost(const GemmF32Args& g, int tile_n, int splits, int sms) {
   const long long items = static_cast<long long>((g.m + 127) / 128) * ((g.n + tile_n - 1) / tile_n) * splits;
-  const long long blocks = ((g.k + 63) / 64 + splits - 1) / splits, waves = (items + SmCount() - 1) / SmCount();
+  const long long blocks = ((g.k + 63) / 64 + splits - 1) / splits, waves = (items + sms - 1) / sms;
   return 4.5 + waves * (0.8 + blocks * (tile_n == 128 ? 2.2 : 1.95)) + ReduceCost(g, splits);
 }
 
+// The cheaper kernel by the estimates above: columns per tile of the tensor-core kernel (0: the CUDA cores) and k splits.
+// Both sides as measured (us, FFMA / tensor cores): [20, 600] x 200 14.7 / 13.4, [595, 450] x 150 12.8 / 12.6, [256, 1536]
+// x 512 27 / 12.2 (4 k splits), [1500, 600] x 300 33 / 15.6, [400, 10000] x 200 84 / 36, [14474, 2048] x 512 1204 / 258;
+// below one 64-wide k block the FFMA kernel is ahead.
+struct Choice { int tile_n, splits; double us; };
+Choice Choose(const GemmF32Args& g) {
+  const long long tiles = static_cast<long long>((g.n + kTN - 1) / kTN) * ((g.m + kTM - 1) / kTM);
+  const int sms = SmCount(), plain = PlainSplits(g, tiles, sms);
+  Choice c{0, plain, PlainCost(g, tiles, plain, sms)};
+  for (int tile : {128, 64})
+    for (int z = 1; z <= 32 && g.k > 0; z *= 2) {
+      if (z > 1 && (g.scratch_bytes == 0 || z > (g.k + 63) / 64 || static_cast<size_t>(z) * g.m * g.n * sizeof(float) > g.scratch_bytes)) break;
+      const double us = SplitCost(g, tile, z, sms);
+      if (us < c.us) c = {tile, z, us};
+    }
+  return c;
+}
+
 }  // namespace
+
+double GemmF32Us(int m, int n, int k, size_t scratch_bytes) {
+  GemmF32Args g;
+  g.m = m; g.n = n; g.k = k;
+  g.scratch_bytes = scratch_bytes;
+  return Choose(g).us;
+}
 
 int GemmF32(const GemmF32Args& g_in, cudaStream_t stream) {
   GemmF32Args g = g_in;
@@ -147,23 +172,12 @@ int GemmF32(const GemmF32Args& g_in, cudaStream_t stream) {
   if (g.m == 0 || g.n == 0) return CAVS_OK;
   CAVS_REQUIRE(g.a && g.b && g.c, CAVS_ERR_BAD_ARG, "gemm_f32: null pointer");
   dim3 grid((g.n + kTN - 1) / kTN, (g.m + kTM - 1) / kTM);
-  const long long tiles = static_cast<long long>(grid.x) * grid.y;
-  int splits = PlainSplits(g, tiles);
-  // The cheaper kernel by the estimates above.  Both sides as measured (us, FFMA / tensor cores): [20, 600] x 200 14.7 /
-  // 13.4, [595, 450] x 150 12.8 / 12.6, [256, 1536] x 512 27 / 12.2 (4 k splits), [1500, 600] x 300 33 / 15.6, [400, 10000]
-  // x 200 84 / 36, [14474, 2048] x 512 1204 / 258; below one 64-wide k block the FFMA kernel is ahead.
-  int tc_tile = 0, tc_splits = 1;
-  double best = PlainCost(g, tiles, splits);
-  for (int tile : {128, 64})
-    for (int z = 1; z <= 32 && g.k > 0; z *= 2) {
-      if (z > 1 && (g.scratch == nullptr || z > (g.k + 63) / 64 || static_cast<size_t>(z) * g.m * g.n * sizeof(float) > g.scratch_bytes)) break;
-      const double cost = SplitCost(g, tile, z);
-      if (cost < best) { best = cost; tc_tile = tile; tc_splits = z; }
-    }
+  if (g.scratch == nullptr) g.scratch_bytes = 0;
+  const Choice choice = Choose(g);
+  int splits = choice.splits;
   g.k_per_split = 0;
-  if (tc_tile > 0) {
-    splits = tc_splits;
-    if (int rc = GemmF32Split(g, tc_tile, &splits, stream)) return rc;
+  if (choice.tile_n > 0) {
+    if (int rc = GemmF32Split(g, choice.tile_n, &splits, stream)) return rc;
   } else {
     if (splits > 1) {
       g.k_per_split = ((g.k + splits - 1) / splits + kTK - 1) / kTK * kTK;

@@ -10,7 +10,7 @@
 namespace cavs_b200 {
 
 // How a range of levels is cut over CTAs: col_groups x row_groups of them, w hidden units each.  w == 0: these sizes
-// do not fit.  level_us: estimated time of a level of `rows` rows.
+// do not fit.  level_us: what the bf16 plan was chosen by, an upper estimate of a level's time.
 struct NarrowPlan {
   int w = 0, col_groups = 0, row_groups = 0, buffers = 0;
   size_t smem = 0;
@@ -18,6 +18,8 @@ struct NarrowPlan {
 };
 NarrowPlan PlanNarrowF32(int H, int K, int rows, bool backward);
 NarrowPlan PlanNarrowBf16(int H, int K, int rows, bool backward);
+// Estimated microseconds of an fp32 level under a plan.
+double NarrowLevelUsF32(const NarrowPlan& plan, int H, int K, int rows, bool backward);
 
 // Levels [level_begin, level_end) in ascending order; level_off: device copy of the level offsets.  Arrays as for the
 // per-level launches (kernels/cell.h): S / HK, the saved gates and h|c of every row are written.  A, S, HK and the

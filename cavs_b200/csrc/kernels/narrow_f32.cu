@@ -442,16 +442,16 @@ int BackwardK(const NarrowBackwardArgs& a, int grid, size_t smem, cudaStream_t s
 NarrowPlan PlanNarrowF32(int H, int K, int rows, bool backward) {
   NarrowPlan best;
   const int tr = K <= 2 ? 32 : 16;
-  const int tiles = (rows + tr - 1) / tr;
+  const int tiles = (rows + tr - 1) / tr, sms = SmCount();
   double best_cost = 0.0;
   for (int w : {4, 8, 16})
    for (int groups : {1, 2}) {   // one row group, or as many as fit
     const int cols = (H + w - 1) / w;
-    if (cols > SmCount()) continue;
+    if (cols > sms) continue;
     NarrowPlan p;
     p.w = w;
     p.col_groups = cols;
-    p.row_groups = groups == 1 ? 1 : std::min(SmCount() / cols, tiles);
+    p.row_groups = groups == 1 ? 1 : std::min(sms / cols, tiles);
     p.buffers = 3 + K;
     if (backward) {
       while (p.buffers > 0 && BackwardSmem(H, K, w, p.buffers) > kMaxSmem) --p.buffers;
@@ -472,8 +472,25 @@ NarrowPlan PlanNarrowF32(int H, int K, int rows, bool backward) {
     const double cost = (p.buffers > 1 ? load + mine * std::max(work, 0.6 * load) : mine * (load + work)) + (backward && p.row_groups > 1 ? 2.5 : 0.0);
     if (best.w == 0 || cost < best_cost) { best = p; best_cost = cost; }
   }
-  best.level_us = 3.0 + best_cost;
   return best;
+}
+
+// Fitted to what levels of 1 to 8192 rows took inside chains of such levels, H = 32 .. 512 and one, two and four child slots
+// (root mean square error 11 % forward, 13 % backward; 10 % where the per-level launches take as long).  A CTA takes every
+// row_groups-th row tile; a level costs its barrier and round trips, each tile in sequence, the rows and multiply-adds of
+// a CTA, rows of no whole 16-byte words (read through registers), and the grid's rows together; backward also the second
+// barrier, a thread's rows of gate gradients and the vectors that find no buffer.
+double NarrowLevelUsF32(const NarrowPlan& p, int H, int K, int rows, bool backward) {
+  const int tr = K <= 2 ? 32 : 16, vectors = 3 + K, read = backward ? vectors : K, tiles = (rows + tr - 1) / tr;
+  const int mine = (tiles + p.row_groups - 1) / p.row_groups;
+  const double mb = 4e-6 * std::min(rows, mine * tr) * H * read, mac = 1e-6 * mine * tr * p.w * H * vectors;
+  const double runs = (H % 4 == 0 ? 0 : H % 2 == 0 ? 1 : 2) * 1e-3 * mine * read * H, all = 1e-3 * rows * vectors;
+  if (!backward) return 1.35 + mine * (1.97 + 0.185 * K) + 22.1 * mb + (p.w == 4 ? 4.6 : 7.4) * mac + 3.0 * runs + 0.14 * all;
+  const bool local = p.row_groups == 1;
+  const int cols = local ? p.w : narrow::kColBlock, strips = local ? 1 : std::max(1, p.col_groups * p.row_groups / ((H + cols - 1) / cols));
+  const int step = strips * (kThreads / cols);
+  return 0.33 + mine * (3.3 + 0.48 * K) + 11.3 * mb + (p.w == 4 ? 1.15 : 8.8) * mac + 3.85 * runs + 1.04 * all + (local ? 0.0 : 2.5) +
+         1.3 * ((rows + step - 1) / step) + 0.97 * mine * std::max(0, vectors - p.buffers);
 }
 
 int LaunchNarrowForwardF32(const NarrowPlan& plan, NarrowForwardArgs a, int K, cudaStream_t st) {
