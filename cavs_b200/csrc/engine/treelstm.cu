@@ -461,7 +461,7 @@ std::vector<NarrowRange> NarrowLevels(const cavs_treelstm* e, const cavs_treelst
       out.push_back({split, n, low});
     }
   }
-  if (!e->bf16) {   // the launches have to pay (the narrower a level the more it saves: the rest is gain then)
+  if (!e->bf16 && n - begin <= 2) {   // the launches have to pay (three levels do: the narrower, the more a level saves)
     double gain = -9.0 * out.size();
     for (const NarrowRange& r : out)
       for (int l = r.begin; l < r.end && gain <= 0.0; ++l) gain += PerLevelUsF32(e, rows(l), backward) - NarrowLevelUsF32(r.plan, H, K, rows(l), backward);

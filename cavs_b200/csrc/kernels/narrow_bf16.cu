@@ -197,7 +197,7 @@ __global__ void __launch_bounds__(kThreads, 1) NarrowForwardBf16(const NarrowFor
     if (l + 1 < a.level_end) {
       GridArrive(a.barrier);
       prefetch(off, end, rg);
-      if (!GridWait(a.barrier, ++barrier * gridDim.x + a.withhold, a.status)) break;
+      if (!GridWait(a.barrier, ++barrier * gridDim.x + a.withhold, a.status)) return;
     }
   }
 }
@@ -239,7 +239,7 @@ __global__ void __launch_bounds__(kThreads, 1) NarrowBackwardBf16(const NarrowBa
     gg.Level(a, off, end);
     GridArrive(a.barrier);
     if (l > a.level_begin) gg.Request(a, next_off, off);   // only the mailbox rows are not complete yet
-    if (!GridWait(a.barrier, ++barrier * gridDim.x + a.withhold, a.status)) break;
+    if (!GridWait(a.barrier, ++barrier * gridDim.x + a.withhold, a.status)) { ring.Drain(); return; }
     const int tiles = (end - off + TR - 1) / TR;
     for (int tile = rg; tile < tiles; tile += a.row_groups) {
       const int t0 = off + tile * TR, rows = min(TR, end - t0);
@@ -315,7 +315,7 @@ __global__ void __launch_bounds__(kThreads, 1) NarrowBackwardBf16(const NarrowBa
       __syncthreads();   // the next level's rows of these columns were written by this CTA
     } else if (l > a.level_begin) {
       GridArrive(a.barrier);
-      if (!GridWait(a.barrier, ++barrier * gridDim.x + a.withhold, a.status)) break;
+      if (!GridWait(a.barrier, ++barrier * gridDim.x + a.withhold, a.status)) { ring.Drain(); return; }
     }
   }
   gg.FoldSums(a, red);

@@ -253,7 +253,7 @@ __global__ void __launch_bounds__(kThreads, 1) NarrowForward(const NarrowForward
     if (l + 1 < a.level_end) {
       GridArrive(a.barrier);
       prefetch(off, end, rg);
-      if (!GridWait(a.barrier, ++barrier * gridDim.x + a.withhold, a.status)) break;
+      if (!GridWait(a.barrier, ++barrier * gridDim.x + a.withhold, a.status)) { ring.Drain(); return; }
     }
   }
   ring.Drain();
@@ -392,7 +392,7 @@ __global__ void __launch_bounds__(kThreads, 1) NarrowBackward(const NarrowBackwa
     gg.Level(a, off, end);
     GridArrive(a.barrier);
     if (l > a.level_begin) gg.Request(a, next_off, off);   // only the mailbox rows are not complete yet
-    if (!GridWait(a.barrier, ++barrier * gridDim.x + a.withhold, a.status)) break;
+    if (!GridWait(a.barrier, ++barrier * gridDim.x + a.withhold, a.status)) { ring.Drain(); return; }
     const int tiles = (end - off + TR - 1) / TR;
     for (int tile = rg; tile < tiles; tile += a.row_groups) {
       const int t0 = off + tile * TR, rows = min(TR, end - t0);
@@ -404,7 +404,7 @@ __global__ void __launch_bounds__(kThreads, 1) NarrowBackward(const NarrowBackwa
       __syncthreads();   // the next level's rows of these columns were written by this CTA
     } else if (l > a.level_begin) {
       GridArrive(a.barrier);
-      if (!GridWait(a.barrier, ++barrier * gridDim.x + a.withhold, a.status)) break;
+      if (!GridWait(a.barrier, ++barrier * gridDim.x + a.withhold, a.status)) { ring.Drain(); return; }
     }
   }
   gg.FoldSums(a, red);
