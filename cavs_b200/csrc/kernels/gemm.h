@@ -122,6 +122,8 @@ struct GemmF32Args {
   int k_per_split = 0;   // set by GemmF32 (0: no split)
 };
 int GemmF32(const GemmF32Args& args, cudaStream_t stream);
+// The same with the kernel given: tile_n 0 the CUDA cores, 64 or 128 the tensor cores; k cut into at most `splits` parts.
+int GemmF32Tiled(const GemmF32Args& args, int tile_n, int splits, cudaStream_t stream);
 // Estimated microseconds of a product with `scratch_bytes` of scratch (the estimate by which GemmF32 chooses its kernel).
 double GemmF32Us(int m, int n, int k, size_t scratch_bytes);
 // The tensor-core kernel alone: tiles of 128 x tile_n (128 or 64).  k is cut over *splits CTAs per tile (rewritten with

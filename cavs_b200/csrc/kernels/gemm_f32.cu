@@ -157,28 +157,19 @@ Choice Choose(const GemmF32Args& g) {
   return c;
 }
 
-}  // namespace
-
-double GemmF32Us(int m, int n, int k, size_t scratch_bytes) {
-  GemmF32Args g;
-  g.m = m; g.n = n; g.k = k;
-  g.scratch_bytes = scratch_bytes;
-  return Choose(g).us;
+int Check(const GemmF32Args& g) {
+  CAVS_REQUIRE(g.m >= 0 && g.n >= 0 && g.k >= 0, CAVS_ERR_BAD_ARG, "gemm_f32: negative dimension");
+  CAVS_REQUIRE(g.m == 0 || g.n == 0 || (g.a && g.b && g.c), CAVS_ERR_BAD_ARG, "gemm_f32: null pointer");
+  return CAVS_OK;
 }
 
-int GemmF32(const GemmF32Args& g_in, cudaStream_t stream) {
+int Run(const GemmF32Args& g_in, int tile_n, int splits, cudaStream_t stream) {
   GemmF32Args g = g_in;
-  CAVS_REQUIRE(g.m >= 0 && g.n >= 0 && g.k >= 0, CAVS_ERR_BAD_ARG, "gemm_f32: negative dimension");
-  if (g.m == 0 || g.n == 0) return CAVS_OK;
-  CAVS_REQUIRE(g.a && g.b && g.c, CAVS_ERR_BAD_ARG, "gemm_f32: null pointer");
-  dim3 grid((g.n + kTN - 1) / kTN, (g.m + kTM - 1) / kTM);
-  if (g.scratch == nullptr) g.scratch_bytes = 0;
-  const Choice choice = Choose(g);
-  int splits = choice.splits;
   g.k_per_split = 0;
-  if (choice.tile_n > 0) {
-    if (int rc = GemmF32Split(g, choice.tile_n, &splits, stream)) return rc;
+  if (tile_n > 0) {
+    if (int rc = GemmF32Split(g, tile_n, &splits, stream)) return rc;
   } else {
+    dim3 grid((g.n + kTN - 1) / kTN, (g.m + kTM - 1) / kTM);
     if (splits > 1) {
       g.k_per_split = ((g.k + splits - 1) / splits + kTK - 1) / kTK * kTK;
       splits = (g.k + g.k_per_split - 1) / g.k_per_split;
@@ -195,6 +186,34 @@ int GemmF32(const GemmF32Args& g_in, cudaStream_t stream) {
   return CAVS_OK;
 }
 
+}  // namespace
+
+double GemmF32Us(int m, int n, int k, size_t scratch_bytes) {
+  GemmF32Args g;
+  g.m = m; g.n = n; g.k = k;
+  g.scratch_bytes = scratch_bytes;
+  return Choose(g).us;
+}
+
+int GemmF32(const GemmF32Args& g_in, cudaStream_t stream) {
+  GemmF32Args g = g_in;
+  if (int rc = Check(g)) return rc;
+  if (g.m == 0 || g.n == 0) return CAVS_OK;
+  if (g.scratch == nullptr) g.scratch_bytes = 0;
+  const Choice c = Choose(g);
+  return Run(g, c.tile_n, c.splits, stream);
+}
+
+int GemmF32Tiled(const GemmF32Args& g, int tile_n, int splits, cudaStream_t stream) {
+  if (int rc = Check(g)) return rc;
+  CAVS_REQUIRE(tile_n == 0 || ((tile_n == 64 || tile_n == 128) && g.k > 0), CAVS_ERR_BAD_ARG,
+               "gemm_f32_tiled: tile_n must be 0, or 64 or 128 with k >= 1");
+  CAVS_REQUIRE(splits == 1 || (splits > 1 && g.k > 0 && g.scratch != nullptr && static_cast<size_t>(splits) * g.m * g.n * sizeof(float) <= g.scratch_bytes),
+               CAVS_ERR_BAD_ARG, "gemm_f32_tiled: k splits need scratch for splits x m x n floats");
+  if (g.m == 0 || g.n == 0) return CAVS_OK;
+  return Run(g, tile_n, splits, stream);
+}
+
 }  // namespace cavs_b200
 
 extern "C" int cavs_gemm_f32(float* c, long long ldc, int accumulate, const float* a, long long a_row_stride,
@@ -206,4 +225,28 @@ extern "C" int cavs_gemm_f32(float* c, long long ldc, int accumulate, const floa
   g.b = b; g.b_rs = b_row_stride; g.b_cs = b_col_stride;
   g.m = m; g.n = n; g.k = k;
   return cavs_b200::GemmF32(g, static_cast<cudaStream_t>(stream));
+}
+
+extern "C" int cavs_gemm_f32_tiled(float* c, long long ldc, int accumulate, const float* a, long long a_row_stride,
+                                   long long a_col_stride, const float* b, long long b_row_stride, long long b_col_stride, int m,
+                                   int n, int k, int tile_n, int splits, float* scratch, size_t scratch_bytes, void* stream) {
+  cavs_b200::GemmF32Args g;
+  g.c = c; g.ldc = ldc; g.accumulate = accumulate;
+  g.a = a; g.a_rs = a_row_stride; g.a_cs = a_col_stride;
+  g.b = b; g.b_rs = b_row_stride; g.b_cs = b_col_stride;
+  g.m = m; g.n = n; g.k = k;
+  g.scratch = scratch; g.scratch_bytes = scratch_bytes;
+  return cavs_b200::GemmF32Tiled(g, tile_n, splits, static_cast<cudaStream_t>(stream));
+}
+
+extern "C" int cavs_gemm_f32_choice(int m, int n, int k, size_t scratch_bytes, int* tile_n, int* splits) {
+  using namespace cavs_b200;
+  CAVS_REQUIRE(m > 0 && n > 0 && k >= 0 && tile_n && splits, CAVS_ERR_BAD_ARG, "gemm_f32_choice: bad argument");
+  GemmF32Args g;
+  g.m = m; g.n = n; g.k = k;
+  g.scratch_bytes = scratch_bytes;
+  const Choice c = Choose(g);
+  *tile_n = c.tile_n;
+  *splits = c.splits;
+  return CAVS_OK;
 }

@@ -4,12 +4,18 @@
 // fp32.
 //
 // Precision.  The tensor core's additions into an accumulator truncate, so a long chain of them would drift where
-// FFMA's rounded additions do not.  Two measures keep the result at least as close to 64 bits as the FFMA kernel's:
-// the leading products hh have an accumulator of their own that takes only the four MMAs of one 64-wide k block and is
-// then added, rounded, to a register; the five correction products, 2^-8 of the size, share a second accumulator
-// that is drained every 512 k.
-//   |err| / |C| against 64 bits (2-norm), normal operands, FFMA kernel -> this one:
-//   k = 150: 2.2e-7 -> 7.6e-8;  k = 512: 4.1e-7 -> 9.0e-8;  k = 2048: 8.1e-7 -> 1.3e-7;  k = 14474: 2.2e-6 -> 3.0e-7.
+// FFMA's rounded additions do not.  Two measures keep the result close to 64 bits: the leading products hh have an
+// accumulator of their own that takes only the four MMAs of one 64-wide k block and is then added, rounded, to a register;
+// the five correction products, 2^-8 of the size, share a second accumulator that is drained every 512 k.
+//   |err| / |C| against 64 bits (2-norm), FFMA kernel -> this one:
+//   normal values         k = 16: 7.4e-8 -> 3.6e-8;  150: 2.2e-7 -> 7.6e-8;  512: 4.1e-7 -> 9.0e-8;  14474: 2.2e-6 -> 3.0e-7
+//   uniform in 0..1       k = 16: 6.2e-8 -> 3.8e-8;   64: 1.2e-7 -> 8.2e-8;  512: 3.1e-7 -> 8.6e-8;  14474: 1.7e-6 -> 2.4e-7
+//   half-normal           k = 16: 6.2e-8 -> 3.9e-8;   64: 1.2e-7 -> 8.9e-8;  512: 3.5e-7 -> 9.6e-8;  14474: 1.8e-6 -> 2.6e-7
+//   sigmoids of normal    k = 16: 6.1e-8 -> 2.7e-8;   64: 1.1e-7 -> 4.1e-8;  512: 3.0e-7 -> 5.6e-8;  14474: 1.7e-6 -> 2.3e-7
+// (of one sign, the truncation is a bias of -1.5e-8 to -8e-8).  Further off than the FFMA kernel where few terms of one sign
+// make up a sum over a short k -- exp(2 x normal): k = 8: 4.2e-8 -> 1.0e-7; 64: 1.9e-7 -> 4.9e-7; closer again from 512 on --
+// where all values lie within 1 % of 2 at k = 14474 (1.7e-6 -> 1.8e-6), and where results lie below 2^-120, whose corrections
+// reach fp32's subnormals (2^-124: 4.0e-7 -> 4.6e-7).
 //
 // What bounds it: 132 TFLOP/s of fp32 products at [14474, 512] x [512, 10000] (5800 us with the FFMA kernel, 1124 with
 // this one), 111 with k = 10000, 99 with k = 14474 and both operands strided along k.  Six MMAs per product stand
@@ -25,8 +31,9 @@
 //                MMAs, one block ahead of the drain (a seventeenth warp would cut every thread to 96 registers)
 //   warps 8..15  operands: global -> registers -> three bf16 planes in 128-byte-swizzled shared memory
 //
-// A value that has no finite split (infinity, NaN, beyond bf16's largest) marks its tile, which is then computed by the
-// plain fp32 loop: such operands give what fp32 arithmetic gives.  So does a tile whose bounded waits expire.
+// A value that its three parts do not hold -- infinity, NaN, beyond bf16's largest, or below 2^-110 with bits that reach under
+// bf16's smallest subnormal, 2^-133 -- marks its tile, which is then computed by the plain fp32 loop: such operands give what
+// fp32 arithmetic gives.  So does a tile whose bounded waits expire.
 #include <cuda_bf16.h>
 
 #include <cstdint>
@@ -100,9 +107,10 @@ __device__ __forceinline__ bool SeekItem(const SplitParams& p, int n_work, int t
 
 __device__ __forceinline__ uint32_t Bits(__nv_bfloat162 x) { return *reinterpret_cast<uint32_t*>(&x); }
 
-// Splits eight values and stores them as one 16-byte word of each plane.  `nan` collects the third parts: a value
-// without a finite split leaves NaN there (infinity - infinity).
-__device__ __forceinline__ void StoreSplit(const float (&v)[8], uint32_t dst, int plane_bytes, __nv_bfloat162& nan) {
+// Splits eight values and stores them as one 16-byte word of each plane.  `rest` collects the bits of what the third part
+// has to hold: those below bf16's sixteen are set when it cannot (a value without a finite split leaves NaN there, infinity -
+// infinity).  One three-input OR per pair of values.
+__device__ __forceinline__ void StoreSplit(const float (&v)[8], uint32_t dst, int plane_bytes, uint32_t& rest) {
   uint32_t h[4], m[4], l[4];
 #pragma unroll
   for (int e = 0; e < 4; ++e) {
@@ -111,8 +119,8 @@ __device__ __forceinline__ void StoreSplit(const float (&v)[8], uint32_t dst, in
     x -= __low2float(hi); y -= __high2float(hi);
     const __nv_bfloat162 mid = __floats2bfloat162_rn(x, y);
     x -= __low2float(mid); y -= __high2float(mid);
+    rest |= __float_as_uint(x) | __float_as_uint(y);
     const __nv_bfloat162 lo = __floats2bfloat162_rn(x, y);
-    nan = __hmax2_nan(nan, lo);
     h[e] = Bits(hi); m[e] = Bits(mid); l[e] = Bits(lo);
   }
   asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(dst), "r"(h[0]), "r"(h[1]), "r"(h[2]), "r"(h[3]) : "memory");
@@ -178,12 +186,12 @@ struct OperandTile {
       }
     }
   }
-  __device__ __forceinline__ void Store(uint32_t dst, int tid, __nv_bfloat162& nan) const {
+  __device__ __forceinline__ void Store(uint32_t dst, int tid, uint32_t& rest) const {
 #pragma unroll
     for (int c = 0; c < kChunks; ++c) {
       int r, j;
       Pos(tid, c, r, j);
-      StoreSplit(v[c], dst + r * 128 + ((j ^ (r & 7)) << 4), kRows * 128, nan);
+      StoreSplit(v[c], dst + r * 128 + ((j ^ (r & 7)) << 4), kRows * 128, rest);
     }
   }
 };
@@ -226,7 +234,7 @@ __global__ void __launch_bounds__(kF32Threads, 1) GemmF32SplitKernel(const Split
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + S::kBarOff);
   uint64_t *full = bars, *empty = bars + 2, *main_full = bars + 4, *main_empty = bars + 6, *corr_empty = bars + 8;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 10);
-  volatile int* marked = reinterpret_cast<volatile int*>(bars + 11);   // [8]: 1 + the tile whose operands have no finite split
+  volatile int* marked = reinterpret_cast<volatile int*>(bars + 11);   // [8]: 1 + the tile with operands that have no exact split
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const GemmF32Args& g = p.g;
@@ -278,13 +286,12 @@ __global__ void __launch_bounds__(kF32Threads, 1) GemmF32SplitKernel(const Split
       ok = WaitPhase(SmemAddr(empty + s), ((it >> 1) & 1) ^ 1);
       if (!ok) break;
       const uint32_t a_dst = SmemAddr(smem + s * S::kStage), b_dst = a_dst + 3 * S::kAPlane;
-      __nv_bfloat162 nan = __floats2bfloat162_rn(0.0f, 0.0f);
-      ta.Store(a_dst, tid, nan);
+      uint32_t rest_a = 0, rest_b = 0;
+      ta.Store(a_dst, tid, rest_a);
       ta.Load(g.a, g.a_rs, g.a_cs, nxt.m0, g.m, nxt.k0, g.k, tid);
-      tb.Store(b_dst, tid, nan);
+      tb.Store(b_dst, tid, rest_b);
       tb.Load(g.b, g.b_cs, g.b_rs, nxt.n0, g.n, nxt.k0, g.k, tid);
-      const float n0 = __low2float(nan), n1 = __high2float(nan);
-      if (n0 != n0 || n1 != n1) marked[t_local & 7] = t_local + 1;
+      if (((rest_a | rest_b) & 0xffffu) != 0) marked[t_local & 7] = t_local + 1;
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
       __syncwarp();
       if (lane == 0) MbarArrive(SmemAddr(full + s));

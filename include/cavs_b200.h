@@ -149,12 +149,21 @@ CAVS_API size_t cavs_gemm_bf16_scratch_bytes(int m, int n, int splits);
  * kernels never wait on one another. */
 CAVS_API int cavs_gemm_bf16_wait_selftest(void* c, long long ldc, const void* a, long long lda, const void* b, long long ldb,
                                           int m, int n, int k, int* status, void* stream);
-/* fp32 GEMM on the CUDA cores with element strides (any transpose without a copy):
+/* fp32 GEMM with element strides (any transpose without a copy), on the tensor cores (operands split into three bf16 parts) or
+ * the CUDA cores, whichever is estimated to be faster:
  * C[i,j] (+)= sum_p A[i*a_row_stride + p*a_col_stride] * B[p*b_row_stride + j*b_col_stride].
  * The fp32 configurations use it to stay within 1e-5 of the reference's cublasSgemm. */
 CAVS_API int cavs_gemm_f32(float* c, long long ldc, int accumulate, const float* a, long long a_row_stride,
                            long long a_col_stride, const float* b, long long b_row_stride, long long b_col_stride, int m,
                            int n, int k, void* stream);
+/* The same with the kernel given, for tests and measurements: tile_n 0 the CUDA cores, 64 or 128 columns per tile of the
+ * tensor-core kernel; k is cut into at most `splits` parts (partial products in scratch, splits * m * n floats, added in
+ * order). */
+CAVS_API int cavs_gemm_f32_tiled(float* c, long long ldc, int accumulate, const float* a, long long a_row_stride,
+                                 long long a_col_stride, const float* b, long long b_row_stride, long long b_col_stride, int m,
+                                 int n, int k, int tile_n, int splits, float* scratch, size_t scratch_bytes, void* stream);
+/* What the fp32 GEMM chooses for a product with `scratch_bytes` of scratch (host only; cavs_gemm_f32 itself has none). */
+CAVS_API int cavs_gemm_f32_choice(int m, int n, int k, size_t scratch_bytes, int* tile_n, int* splits);
 
 /* ------------------------------------------------------------------------ */
 /* Fused vertex-function kernels (device).  Level rows are [off, off+rows) of */
