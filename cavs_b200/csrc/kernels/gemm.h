@@ -120,6 +120,7 @@ struct GemmF32Args {
   float* scratch = nullptr;
   size_t scratch_bytes = 0;
   int k_per_split = 0;   // set by GemmF32 (0: no split)
+  int withhold = 0;      // self-test of the tensor-core kernel's bounded waits: no operand is ever ready, all of them expire
 };
 int GemmF32(const GemmF32Args& args, cudaStream_t stream);
 // The same with the kernel given: tile_n 0 the CUDA cores, 64 or 128 the tensor cores; k cut into at most `splits` parts.

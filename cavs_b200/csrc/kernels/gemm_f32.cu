@@ -229,13 +229,13 @@ extern "C" int cavs_gemm_f32(float* c, long long ldc, int accumulate, const floa
 
 extern "C" int cavs_gemm_f32_tiled(float* c, long long ldc, int accumulate, const float* a, long long a_row_stride,
                                    long long a_col_stride, const float* b, long long b_row_stride, long long b_col_stride, int m,
-                                   int n, int k, int tile_n, int splits, float* scratch, size_t scratch_bytes, void* stream) {
+                                   int n, int k, int tile_n, int splits, int withhold, float* scratch, size_t scratch_bytes, void* stream) {
   cavs_b200::GemmF32Args g;
   g.c = c; g.ldc = ldc; g.accumulate = accumulate;
   g.a = a; g.a_rs = a_row_stride; g.a_cs = a_col_stride;
   g.b = b; g.b_rs = b_row_stride; g.b_cs = b_col_stride;
   g.m = m; g.n = n; g.k = k;
-  g.scratch = scratch; g.scratch_bytes = scratch_bytes;
+  g.scratch = scratch; g.scratch_bytes = scratch_bytes; g.withhold = withhold;
   return cavs_b200::GemmF32Tiled(g, tile_n, splits, static_cast<cudaStream_t>(stream));
 }
 

@@ -68,6 +68,7 @@ struct SplitParams {
   int n_splits, kb_per_split;
   long long split_stride;
   int chain_early;
+  int withhold;   // wait self-test: no operand is ever ready
 };
 
 // Bounded wait (about 0.3 s) whose polls suspend the warp in hardware, so that waiting warps leave the issue slots to
@@ -79,6 +80,23 @@ __device__ __forceinline__ bool WaitPhase(uint32_t bar, uint32_t parity) {
         "{\n\t.reg .pred p;\n\t"
         "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, 1000;\n\t"
         "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(done)
+        : "r"(bar), "r"(parity)
+        : "memory");
+    if (done) return true;
+  }
+  return false;
+}
+// The same by a whole warp, with one outcome for all lanes: warp-wide instructions follow.  (The vote stands inside the poll:
+// a vote on the outcome cost 100 bytes of spilled registers.)
+__device__ __forceinline__ bool WaitPhaseWarp(uint32_t bar, uint32_t parity) {
+  for (uint32_t it = 0; it < (1u << 18); ++it) {
+    uint32_t done;
+    asm volatile(
+        "{\n\t.reg .pred p, q;\n\t"
+        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, 1000;\n\t"
+        "vote.sync.all.pred q, p, 0xffffffff;\n\t"
+        "selp.u32 %0, 1, 0, q;\n\t}"
         : "=r"(done)
         : "r"(bar), "r"(parity)
         : "memory");
@@ -232,9 +250,9 @@ __global__ void __launch_bounds__(kF32Threads, 1) GemmF32SplitKernel(const Split
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + S::kBarOff);
-  uint64_t *full = bars, *empty = bars + 2, *main_full = bars + 4, *main_empty = bars + 6, *corr_empty = bars + 8;
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 10);
-  volatile int* marked = reinterpret_cast<volatile int*>(bars + 11);   // [8]: 1 + the tile with operands that have no exact split
+  uint64_t *full = bars, *empty = bars + 2, *main_full = bars + 4, *main_empty = bars + 6, *corr_empty = bars + 8, *drained = bars + 10;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 11);
+  volatile int* marked = reinterpret_cast<volatile int*>(bars + 12);   // [8]: 1 + the tile with operands that have no exact split
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const GemmF32Args& g = p.g;
@@ -248,6 +266,7 @@ __global__ void __launch_bounds__(kF32Threads, 1) GemmF32SplitKernel(const Split
       MbarInit(SmemAddr(main_empty + s), kDrainWarps);
       MbarInit(SmemAddr(corr_empty + s), kDrainWarps);
     }
+    MbarInit(SmemAddr(drained), 1);
     for (int i = 0; i < 8; ++i) marked[i] = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
@@ -269,7 +288,7 @@ __global__ void __launch_bounds__(kF32Threads, 1) GemmF32SplitKernel(const Split
     OperandTile<kBN, kModeB> tb;
     BlockPos nxt;   // the next block to load
     nxt.w = blockIdx.x; nxt.t_local = 0;
-    bool have = SeekItem<kBN>(p, n_work, tiles_n, nxt);   // always: the grid is no larger than the work list
+    bool have = SeekItem<kBN>(p, n_work, tiles_n, nxt) && !p.withhold;   // (the grid is no larger than the work list)
     ta.Load(g.a, g.a_rs, g.a_cs, nxt.m0, g.m, nxt.k0, g.k, tid);
     tb.Load(g.b, g.b_cs, g.b_rs, nxt.n0, g.n, nxt.k0, g.k, tid);
     for (uint32_t it = 0; have; ++it) {
@@ -283,7 +302,7 @@ __global__ void __launch_bounds__(kF32Threads, 1) GemmF32SplitKernel(const Split
         if (!have) nxt.k0 = g.k;   // nothing follows: loads of zeros, so that the loads stand behind no branch
       }
       const int s = it & 1;
-      ok = WaitPhase(SmemAddr(empty + s), ((it >> 1) & 1) ^ 1);
+      ok = WaitPhaseWarp(SmemAddr(empty + s), ((it >> 1) & 1) ^ 1);
       if (!ok) break;
       const uint32_t a_dst = SmemAddr(smem + s * S::kStage), b_dst = a_dst + 3 * S::kAPlane;
       uint32_t rest_a = 0, rest_b = 0;
@@ -356,7 +375,7 @@ __global__ void __launch_bounds__(kF32Threads, 1) GemmF32SplitKernel(const Split
       for (int i = 0; i < b.kb_count && ok; ++i, ++it) {
         const int s = it & 1;
         if (warp == 0) issue_next();   // the block after this one: its MMAs follow this block's without a gap
-        ok = ok && WaitPhase(SmemAddr(main_full + s), (it >> 1) & 1);
+        ok = ok && WaitPhaseWarp(SmemAddr(main_full + s), (it >> 1) & 1);
         if (!ok) break;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         const bool corr_last = i % kCorrBlocks == kCorrBlocks - 1 || i == b.kb_count - 1;
@@ -417,6 +436,13 @@ __global__ void __launch_bounds__(kF32Threads, 1) GemmF32SplitKernel(const Split
         }
       }
     }
+    if (warp == 0 && !ok) {   // the accumulators are given back when no MMA is under way any more
+      if (lane == 0) {
+        UmmaCommit(SmemAddr(drained));
+        WaitPhase(SmemAddr(drained), 0);
+      }
+      __syncwarp();
+    }
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
@@ -474,6 +500,7 @@ int GemmF32Split(const GemmF32Args& g, int tile_n, int* splits, cudaStream_t str
   p.n_splits = *splits = (kb + p.kb_per_split - 1) / p.kb_per_split;
   p.split_stride = static_cast<long long>(g.m) * g.n;
   p.chain_early = ChainEarly();
+  p.withhold = g.withhold;
   const ReadMode ma = ReadModeOf(g.a, g.m, g.a_rs, g.k, g.a_cs, kBM), mb = ReadModeOf(g.b, g.n, g.b_cs, g.k, g.b_rs, tile_n);
   return tile_n == 128 ? LaunchSplitAB<128>(p, ma, mb, stream) : LaunchSplitAB<64>(p, ma, mb, stream);
 }

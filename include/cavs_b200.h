@@ -158,10 +158,11 @@ CAVS_API int cavs_gemm_f32(float* c, long long ldc, int accumulate, const float*
                            int n, int k, void* stream);
 /* The same with the kernel given, for tests and measurements: tile_n 0 the CUDA cores, 64 or 128 columns per tile of the
  * tensor-core kernel; k is cut into at most `splits` parts (partial products in scratch, splits * m * n floats, added in
- * order). */
+ * order).  withhold 1: the kernel's operands never become ready, so that all its bounded waits run out, which costs time
+ * and not the result. */
 CAVS_API int cavs_gemm_f32_tiled(float* c, long long ldc, int accumulate, const float* a, long long a_row_stride,
                                  long long a_col_stride, const float* b, long long b_row_stride, long long b_col_stride, int m,
-                                 int n, int k, int tile_n, int splits, float* scratch, size_t scratch_bytes, void* stream);
+                                 int n, int k, int tile_n, int splits, int withhold, float* scratch, size_t scratch_bytes, void* stream);
 /* What the fp32 GEMM chooses for a product with `scratch_bytes` of scratch (host only; cavs_gemm_f32 itself has none). */
 CAVS_API int cavs_gemm_f32_choice(int m, int n, int k, size_t scratch_bytes, int* tile_n, int* splits);
 

@@ -1,5 +1,5 @@
 """The fp32 GEMM's kernels through cavs_gemm_f32_tiled, each given outright: both tile widths of the tensor-core kernel, k cut over
-CTAs, accumulation, every way of reading an operand, values whose three bf16 parts do not hold them.
+CTAs, accumulation, every way of reading an operand, values whose three bf16 parts do not hold them, waits that run out.
 
 Tolerance, per value and against a 64-bit product: 2^-24 of sum |a||b| for each operation that rounds on the way -- the split
 of the operands and the products kept (8), two for every 64 values of k (the accumulator's additions truncate, its value is
@@ -19,7 +19,7 @@ def _p(t):
     return ctypes.c_void_p(t.data_ptr() if t is not None else 0)
 
 
-def _gemm(A, B, tile_n, splits=1, C0=None):
+def _gemm(A, B, tile_n, splits=1, C0=None, withhold=0):
     m, k = A.shape
     n = B.shape[1]
     C = torch.full((m, n + 5), 7.0, device=A.device)
@@ -27,7 +27,7 @@ def _gemm(A, B, tile_n, splits=1, C0=None):
         C[:, :n] = C0
     scratch = torch.empty(splits * m * n, device=A.device) if splits > 1 else None
     check(lib().cavs_gemm_f32_tiled(_p(C), ll(C.stride(0)), int(C0 is not None), _p(A), ll(A.stride(0)), ll(A.stride(1)), _p(B), ll(B.stride(0)),
-                                    ll(B.stride(1)), m, n, k, tile_n, splits, _p(scratch),
+                                    ll(B.stride(1)), m, n, k, tile_n, splits, withhold, _p(scratch),
                                     ctypes.c_size_t(4 * scratch.numel() if splits > 1 else 0),
                                     ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)))
     torch.cuda.synchronize()
@@ -103,3 +103,14 @@ def test_small_values_keep_their_bits(cuda, tile_n, exponent):
     C = _gemm(A, B, tile_n)
     # (results may lie under fp32's smallest normal value: half a unit of the smallest subnormal for each operation)
     assert bool(((C.double() - A.double() @ B.double()).abs() <= _bound(A, B, k) + k * 2.0**-150).all())
+
+
+@pytest.mark.parametrize("tile_n", [64, 128])
+@pytest.mark.parametrize("splits", [1, 3])
+def test_waits_that_run_out_cost_time_not_the_result(cuda, tile_n, splits):
+    # no operand is ever handed over, so that every wait of the kernel expires: plain fp32 loops give the product
+    g = torch.Generator().manual_seed(9)
+    A, B = torch.randn((200, 200), generator=g).to(cuda), torch.randn((200, 190), generator=g).to(cuda)
+    want = _gemm(A, B, tile_n, splits, withhold=1)
+    assert bool(((want.double() - A.double() @ B.double()).abs() <= _bound(A, B, 200 + splits)).all())
+    assert bool(((_gemm(A, B, tile_n, splits).double() - A.double() @ B.double()).abs() <= _bound(A, B, _rounds(200, splits))).all())
