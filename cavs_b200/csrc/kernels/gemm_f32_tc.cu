@@ -32,8 +32,8 @@
 //   warps 8..15  operands: global -> registers -> three bf16 planes in 128-byte-swizzled shared memory
 //
 // A value that its three parts do not hold -- infinity, NaN, beyond bf16's largest, or below 2^-110 with bits that reach under
-// bf16's smallest subnormal, 2^-133 -- marks its tile, which is then computed by the plain fp32 loop: such operands give what
-// fp32 arithmetic gives.  So does a tile whose bounded waits expire.
+// bf16's smallest subnormal, 2^-133 -- marks its tile, which is computed by plain fp32 loops after all others: such operands give
+// what fp32 arithmetic gives.  So does a tile whose bounded waits expire, row by row.
 #include <cuda_bf16.h>
 
 #include <cstdint>
@@ -51,6 +51,7 @@ using namespace tc;   // mbarrier, TMEM and MMA wrappers of the bf16 GEMM
 constexpr int kDrainWarps = 8, kSplitWarps = 8;
 constexpr int kF32Threads = (kDrainWarps + kSplitWarps) * 32;
 constexpr int kSplitThreads = kSplitWarps * 32;
+constexpr int kMarks = 4096;     // tiles per CTA that can be marked one by one (the last bit stands for all from there on)
 constexpr int kCorrBlocks = 8;   // k blocks per drain of the correction accumulator
 
 template <int kBN>
@@ -60,7 +61,7 @@ struct SplitSmem {
   static constexpr int kStages = 2;
   static constexpr int kCOff = kStages * kStage;
   static constexpr int kBarOff = kCOff + kDrainWarps * 32 * 128;
-  static constexpr int kBytes = kBarOff + 256 + 1024;
+  static constexpr int kBytes = kBarOff + 96 + kMarks / 8 + 1024;   // barriers, TMEM address, marks; alignment
 };
 
 struct SplitParams {
@@ -231,8 +232,9 @@ __device__ __forceinline__ void DrainAdd(float (&acc)[kCols], uint32_t taddr) {
   }
 }
 
-__device__ __noinline__ void PlainTile(const GemmF32Args& g, float* c, long long ldc, int accumulate, int row, int col0, int cols, int k0,
-                                       int k1) {
+// One row of a tile's columns [col0, col0 + cols) in fp32, by one thread that waits for nobody: after an expired wait.
+__device__ __noinline__ void PlainRow(const GemmF32Args& g, float* c, long long ldc, int accumulate, int row, int col0, int cols, int k0,
+                                      int k1) {
   if (row >= g.m) return;
   for (int j = col0; j < min(col0 + cols, g.n); ++j) {
     float acc = 0.0f;
@@ -240,6 +242,89 @@ __device__ __noinline__ void PlainTile(const GemmF32Args& g, float* c, long long
     float* dst = c + row * ldc + j;
     *dst = accumulate ? *dst + acc : acc;
   }
+}
+
+// A whole tile in fp32 by all threads, k ascending: 8 x kBN / 32 outputs per thread in a 16 x 32 grid of threads, 32 k values
+// staged at a time in the operands' shared memory, the next ones in flight meanwhile.
+template <int kBN>
+__device__ __forceinline__ void PlainTile(const GemmF32Args& g, float* c, long long ldc, int accumulate, int m0, int n0, int k0, int k1,
+                                       float* stage) {
+  constexpr int kC = kBN / 32, kStep = 32, kPitchA = kBM + 4, kPitchB = kBN + 4;
+  constexpr int kLoadA = kBM * kStep / kF32Threads, kLoadB = kBN * kStep / kF32Threads;
+  float *as = stage, *bs = stage + kStep * kPitchA;
+  const int tc = threadIdx.x & 31, tr = threadIdx.x >> 5;
+  float acc[8][kC], va[kLoadA], vb[kLoadB];
+#pragma unroll
+  for (int i = 0; i < 8; ++i)
+#pragma unroll
+    for (int j = 0; j < kC; ++j) acc[i][j] = 0.0f;
+  // element e of a thread: neighbouring threads read along the operand's contiguous direction
+  const bool a_k = g.a_cs == 1, b_k = g.b_rs == 1;
+  auto at_a = [&](int e, int& r, int& k) { const int i = threadIdx.x + e * kF32Threads; if (a_k) { k = i % kStep; r = i / kStep; } else { r = i % kBM; k = i / kBM; } };
+  auto at_b = [&](int e, int& j, int& k) { const int i = threadIdx.x + e * kF32Threads; if (b_k) { k = i % kStep; j = i / kStep; } else { j = i % kBN; k = i / kBN; } };
+  auto load = [&](int kb) {
+    int r, k;
+#pragma unroll
+    for (int e = 0; e < kLoadA; ++e) { at_a(e, r, k); va[e] = m0 + r < g.m && kb + k < k1 ? g.a[(m0 + r) * g.a_rs + (kb + k) * g.a_cs] : 0.0f; }
+#pragma unroll
+    for (int e = 0; e < kLoadB; ++e) { at_b(e, r, k); vb[e] = n0 + r < g.n && kb + k < k1 ? g.b[(kb + k) * g.b_rs + (n0 + r) * g.b_cs] : 0.0f; }
+  };
+  load(k0);
+  for (int kb = k0; kb < k1; kb += kStep) {
+    int r, k;
+    __syncthreads();   // the previous values' readers are done
+#pragma unroll
+    for (int e = 0; e < kLoadA; ++e) { at_a(e, r, k); as[k * kPitchA + r] = va[e]; }
+#pragma unroll
+    for (int e = 0; e < kLoadB; ++e) { at_b(e, r, k); bs[k * kPitchB + r] = vb[e]; }
+    __syncthreads();
+    load(kb + kStep);
+#pragma unroll 8
+    for (int u = 0; u < kStep; ++u) {
+      float x[8];
+#pragma unroll
+      for (int i = 0; i < 8; i += 4) {
+        const float4 t = *reinterpret_cast<const float4*>(as + u * kPitchA + tr * 8 + i);
+        x[i] = t.x; x[i + 1] = t.y; x[i + 2] = t.z; x[i + 3] = t.w;
+      }
+#pragma unroll
+      for (int j = 0; j < kC; ++j) {
+        const float y = bs[u * kPitchB + j * 32 + tc];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) acc[i][j] = fmaf(x[i], y, acc[i][j]);
+      }
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < 8; ++i)
+#pragma unroll
+    for (int j = 0; j < kC; ++j) {
+      const int row = m0 + tr * 8 + i, col = n0 + j * 32 + tc;
+      if (row >= g.m || col >= g.n) continue;
+      float* dst = c + row * ldc + col;
+      *dst = accumulate ? *dst + acc[i][j] : acc[i][j];
+    }
+}
+
+// The marked tiles of this CTA, after all others: nobody waits for them then, and a function of its own, called where nothing
+// else is live, leaves the registers of the loops alone.  [14474, 512] x [512, 10000] with every tile marked: 7.3 ms (FFMA
+// kernel 5.7; one thread per row 45 or more), with one marked 1.29 (1.15 without).
+template <int kBN>
+__device__ __noinline__ void PlainTiles(const SplitParams& p) {
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
+  const uint32_t* words = reinterpret_cast<const uint32_t*>(smem + SplitSmem<kBN>::kBarOff) + 23;   // any mark, marks
+  if (words[0] == 0) return;
+  const int tiles_n = (p.g.n + kBN - 1) / kBN, n_work = ((p.g.m + kBM - 1) / kBM) * tiles_n * p.n_splits;
+  for (int i = 0; i < kMarks / 32; ++i)
+    for (uint32_t word = words[1 + i]; word != 0; word &= word - 1) {
+      BlockPos b;
+      b.w = blockIdx.x + (i * 32 + __ffs(word) - 1) * gridDim.x;
+      if (i * 32 + __ffs(word) == kMarks || !SeekItem<kBN>(p, n_work, tiles_n, b)) continue;
+      const bool part = p.n_splits > 1;
+      PlainTile<kBN>(p.g, part ? p.g.scratch + (b.w % p.n_splits) * p.split_stride : p.g.c, part ? p.g.n : p.g.ldc, part ? 0 : p.g.accumulate, b.m0,
+                     b.n0, b.k0, min(p.g.k, b.k0 + b.kb_count * kBK), reinterpret_cast<float*>(smem));
+    }
 }
 
 template <int kBN, int kModeA, int kModeB>
@@ -252,7 +337,8 @@ __global__ void __launch_bounds__(kF32Threads, 1) GemmF32SplitKernel(const Split
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + S::kBarOff);
   uint64_t *full = bars, *empty = bars + 2, *main_full = bars + 4, *main_empty = bars + 6, *corr_empty = bars + 8, *drained = bars + 10;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 11);
-  volatile int* marked = reinterpret_cast<volatile int*>(bars + 12);   // [8]: 1 + the tile with operands that have no exact split
+  uint32_t* any_mark = tmem_slot + 1;
+  uint32_t* marks = reinterpret_cast<uint32_t*>(bars + 12);   // one bit per tile of this CTA with operands that have no exact split
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const GemmF32Args& g = p.g;
@@ -267,9 +353,10 @@ __global__ void __launch_bounds__(kF32Threads, 1) GemmF32SplitKernel(const Split
       MbarInit(SmemAddr(corr_empty + s), kDrainWarps);
     }
     MbarInit(SmemAddr(drained), 1);
-    for (int i = 0; i < 8; ++i) marked[i] = 0;
+    *any_mark = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
+  for (int i = threadIdx.x; i < kMarks / 32; i += kF32Threads) marks[i] = 0;
   if (warp == 0) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(SmemAddr(tmem_slot)), "r"(4 * kBN));
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
@@ -310,7 +397,10 @@ __global__ void __launch_bounds__(kF32Threads, 1) GemmF32SplitKernel(const Split
       ta.Load(g.a, g.a_rs, g.a_cs, nxt.m0, g.m, nxt.k0, g.k, tid);
       tb.Store(b_dst, tid, rest_b);
       tb.Load(g.b, g.b_cs, g.b_rs, nxt.n0, g.n, nxt.k0, g.k, tid);
-      if (((rest_a | rest_b) & 0xffffu) != 0) marked[t_local & 7] = t_local + 1;
+      if (((rest_a | rest_b) & 0xffffu) != 0) {
+        atomicOr(marks + (min(t_local, kMarks - 1) >> 5), 1u << (min(t_local, kMarks - 1) & 31));
+        *any_mark = 1;
+      }
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
       __syncwarp();
       if (lane == 0) MbarArrive(SmemAddr(full + s));
@@ -394,8 +484,10 @@ __global__ void __launch_bounds__(kF32Threads, 1) GemmF32SplitKernel(const Split
       const long long ldc = p.n_splits > 1 ? g.n : g.ldc;
       const int accumulate = p.n_splits > 1 ? 0 : g.accumulate;
       const int row0 = b.m0 + quarter * 32, col_base = b.n0 + half * kCols;
-      if (!ok || marked[b.t_local & 7] == b.t_local + 1) {
-        PlainTile(g, c, ldc, accumulate, row0 + lane, col_base, kCols, b.k0, min(g.k, b.k0 + b.kb_count * kBK));
+      const int mark = min(b.t_local, kMarks - 1);
+      const bool marked = *reinterpret_cast<volatile uint32_t*>(marks + (mark >> 5)) >> (mark & 31) & 1;
+      if (!ok || marked) {   // marked: computed after all others, but for the tiles that share the last bit
+        if (!marked || mark == kMarks - 1) PlainRow(g, c, ldc, accumulate, row0 + lane, col_base, kCols, b.k0, min(g.k, b.k0 + b.kb_count * kBK));
         continue;
       }
       const bool vec = (ldc & 3) == 0 && (reinterpret_cast<uintptr_t>(c) & 15) == 0;
@@ -448,6 +540,7 @@ __global__ void __launch_bounds__(kF32Threads, 1) GemmF32SplitKernel(const Split
   __syncthreads();
   if (warp == 0)
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(4 * kBN));
+  PlainTiles<kBN>(p);
 }
 
 ReadMode ReadModeOf(const float* base, int rows, long long row_stride, int k, long long k_stride, int tile_rows) {

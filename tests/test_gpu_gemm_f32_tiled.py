@@ -106,6 +106,29 @@ def test_small_values_keep_their_bits(cuda, tile_n, exponent):
 
 
 @pytest.mark.parametrize("tile_n", [64, 128])
+@pytest.mark.parametrize("splits,accumulate", [(1, False), (1, True), (3, False)])
+def test_marked_tiles_among_many(cuda, tile_n, splits, accumulate):
+    # several tiles per CTA, some of them computed by plain fp32 loops afterwards, beside ordinary ones
+    g = torch.Generator().manual_seed(tile_n + splits)
+    m, n, k = 2500, 1300, 400
+    A, B = torch.randn((m, k), generator=g), torch.randn((k, n), generator=g)
+    A[3, 5], A[1200, 399], A[2499, 0], A[700, 100] = float("inf"), 1e-39, float("nan"), 3.4e38
+    B[:, 50] = 0
+    B[100] *= 0.01
+    B[17, 1299] = -float("inf")
+    C0 = torch.randn((m, n), generator=g).to(cuda) if accumulate else None
+    A, B = A.to(cuda), B.to(cuda)
+    C = _gemm(A, B, tile_n, splits, C0)
+    R = A.double() @ B.double()
+    if accumulate:
+        R += C0.double()
+    assert torch.equal(torch.isnan(C), torch.isnan(R))
+    assert bool((C[R == float("inf")] == float("inf")).all()) and bool((C[R == -float("inf")] == -float("inf")).all())
+    small = R.abs() < 1e30
+    assert bool(((C.double() - R).abs() <= _bound(A, B, k + splits + 1, C0))[small].all())
+
+
+@pytest.mark.parametrize("tile_n", [64, 128])
 @pytest.mark.parametrize("splits", [1, 3])
 def test_waits_that_run_out_cost_time_not_the_result(cuda, tile_n, splits):
     # no operand is ever handed over, so that every wait of the kernel expires: plain fp32 loops give the product
