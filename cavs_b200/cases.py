@@ -19,6 +19,9 @@ Small, self-contained cases of the library's kernels, sized for profiler capture
     python -m cavs_b200.cases shard   two training steps of the Tree-LSTM engine on one rank's shard of the
                                       benchmark workload at 8 GPUs (512 trees, ~66 k vertices, ~4 GB);
                                       `shard 50` also times 50 further steps with CUDA events
+    python -m cavs_b200.cases product the fp32 product [14474,512] x [512,10000] on the tensor cores, three times (0.6 GB)
+    python -m cavs_b200.cases narrow  three forward + backward passes over narrow levels alone: 96 chains of 5..60 vertices (hidden
+                                      512, bf16), then 20 chains of 20 (hidden 200, fp32)
     python -m cavs_b200.cases unbatched [steps]
                                       what level batching buys: the binary Tree-LSTM configuration (64 trees of 2..50
                                       leaves, hidden 150, embedding 300, fp32) stepped with the level schedule and with the
@@ -201,6 +204,31 @@ def gru(steps: int = 3) -> None:
     print("loss", eng.read_loss(), "vertices", s.n_total, "levels", s.n_levels, "level rows", np.diff(s.level_off).tolist())
 
 
+def product(iters: int = 3) -> None:
+    L, dev, ll = lib(), torch.device("cuda"), ctypes.c_longlong
+    m, n, k = 14474, 10000, 512
+    a, b, c = torch.randn((m, k), device=dev), torch.randn((k, n), device=dev), torch.empty((m, n), device=dev)
+    for _ in range(iters):
+        rc = L.cavs_gemm_f32(_p(c), ll(n), 0, _p(a), ll(k), ll(1), _p(b), ll(n), ll(1), m, n, k, _st())
+        assert rc == 0, L.cavs_last_error()
+    torch.cuda.synchronize()
+
+
+def narrow(steps: int = 3) -> None:
+    import numpy as np
+    for H, bf16, batch, lo, hi in ((512, True, 96, 5, 60), (200, False, 20, 20, 20)):
+        parents = S.synth_chains(5, batch, lo, hi)
+        s = S.Schedule().load(parents, n_slots=1)
+        eng = TreeLSTM(H, 64, 1000, 5, n_slots=1, gemm_bf16=bf16, max_vertices=s.n_total, max_level_rows=s.max_level_rows)
+        eng.params.uniform_(-0.05, 0.05)
+        eng.refresh_weights()
+        eng.load_batch(s, S.synth_zipf(6, 1.1, 1000, s.n_total), S.synth_uniform_int(7, 5, s.n_total))
+        for _ in range(steps):
+            eng.forward()
+            eng.backward()
+        print("loss", eng.read_loss(), "vertices", s.n_total, "levels", s.n_levels, "level rows", np.diff(s.level_off).tolist())
+
+
 def unbatched(steps: int = 10) -> None:
     import numpy as np
     H, E, V, C, batch = 150, 300, 21701, 5, 64
@@ -235,6 +263,7 @@ def unbatched(steps: int = 10) -> None:
 
 
 if __name__ == "__main__":
-    fn = {"gemm": gemm, "loss": loss, "cell": cell, "shard": shard, "unbatched": unbatched, "level": level, "gru": gru, "rows": rows}[sys.argv[1]]
+    fn = {"gemm": gemm, "loss": loss, "cell": cell, "shard": shard, "unbatched": unbatched, "level": level, "gru": gru, "rows": rows, "product": product,
+          "narrow": narrow}[sys.argv[1]]
     fn(*(int(a) for a in sys.argv[2:3]))   # optional iteration / step count
     print("ok", sys.argv[1])

@@ -90,6 +90,16 @@ size_t IdxInts(const cavs_treelstm_config& c) {
   return (c.n_slots + 5) * n + (MaxChunks(c) + 1) + (MaxSegments(c) + 1) + MaxSegments(c) + 64;
 }
 
+// fp32: k-split scratch for every product of a step at full capacity.
+size_t SplitF32Bytes(const cavs_treelstm_config& c) {
+  const size_t N = c.max_vertices, L = c.max_level_rows, T = MaxSegments(c), H = c.hidden, E = c.embed, K = c.n_slots;
+  size_t b = 0;
+  auto need = [&](size_t m, size_t n, size_t k) { b = std::max(b, GemmF32ScratchBytes(m, n, k)); };
+  need(T, 3 * H, E); need(T, E, 3 * H); need(E, 3 * H, T);
+  need(L * K, H, H); need(H, H, N * K);
+  return std::min(b, GemmF32ScratchCap());
+}
+
 size_t Carve(cavs_treegru* e, void* base) {
   const cavs_treelstm_config& c = e->cfg;
   const size_t N = c.max_vertices, L = c.max_level_rows, H = c.hidden, E = c.embed, K = c.n_slots, T = MaxSegments(c);
@@ -122,7 +132,7 @@ size_t Carve(cavs_treegru* e, void* base) {
   e->loss_scratch = w.Take<float>(LossHeadScratchBytes(c.hidden, c.classes) / sizeof(float));
   e->col_scratch = w.Take<float>(ColumnSumScratchBytes(3 * c.hidden) / sizeof(float));
   e->emb_scratch = w.Take<float>(MaxChunks(c) * 3 * H);
-  e->splitk_bytes = c.gemm_bf16 ? std::max(GemmBf16ScratchBytes(c.embed, 3 * c.hidden, 32), GemmBf16ScratchBytes(c.hidden, c.hidden, 32)) : GemmF32ScratchBytes();
+  e->splitk_bytes = c.gemm_bf16 ? std::max(GemmBf16ScratchBytes(c.embed, 3 * c.hidden, 32), GemmBf16ScratchBytes(c.hidden, c.hidden, 32)) : SplitF32Bytes(c);
   e->splitk_scratch = w.Take<float>(e->splitk_bytes / sizeof(float));
   e->W_bf = w.Take<uint8_t>(c.gemm_bf16 ? E * 3 * H * 2 : 0);
   e->U_bf = w.Take<uint8_t>(c.gemm_bf16 ? 3 * H * H * 2 : 0);

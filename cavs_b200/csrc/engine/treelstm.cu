@@ -276,7 +276,15 @@ size_t IdxInts(const cavs_treelstm_config& c) {
 
 // Split-K scratch large enough for the three weight-gradient GEMMs at full capacity.
 size_t SplitKBytes(const cavs_treelstm_config& c) {
-  if (!c.gemm_bf16) return std::max(GemmF32ScratchBytes(), static_cast<size_t>(16) * 64 * 4 * c.hidden * sizeof(float));
+  if (!c.gemm_bf16) {   // every product of a step at full capacity
+    const size_t N = c.max_vertices, L = c.max_level_rows, T = MaxSegments(c), H = c.hidden, E = c.embed, K = c.n_slots, C = c.classes;
+    size_t b = 0;
+    auto need = [&](size_t m, size_t n, size_t k) { b = std::max(b, GemmF32ScratchBytes(m, n, k)); };
+    need(T, 4 * H, E); need(T, E, 4 * H); need(E, 4 * H, T);                                   // input projection and its gradients
+    need(L, 3 * H, H); need(L * K, H, H); need(L, H, 3 * H); need(H, 3 * H, N); need(H, H, N * K);   // recurrent products
+    if (C > 8) { need(N, C, H); need(N, H, C); need(C, H, N); }                                // wide loss head
+    return std::min(b, std::max(GemmF32ScratchCap(), static_cast<size_t>(16) * 64 * 4 * H * sizeof(float)));
+  }
   const int N = c.max_vertices, H = c.hidden, E = c.embed, K = c.n_slots;
   size_t b = GemmBf16ScratchBytes(E, 4 * H, 32);
   b = std::max(b, GemmBf16ScratchBytes(H, 3 * H, 32));

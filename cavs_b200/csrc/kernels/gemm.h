@@ -130,8 +130,10 @@ double GemmF32Us(int m, int n, int k, size_t scratch_bytes);
 // The tensor-core kernel alone: tiles of 128 x tile_n (128 or 64).  k is cut over *splits CTAs per tile (rewritten with
 // the number used); with more than one the partial products are left in args.scratch [splits, m, n].
 int GemmF32Split(const GemmF32Args& args, int tile_n, int* splits, cudaStream_t stream);
-// Scratch with which no product of a step is short of k splits: two partial tiles per SM.
-inline size_t GemmF32ScratchBytes() { return static_cast<size_t>(2) * 148 * 128 * 128 * sizeof(float); }
+// Scratch with which an [m, n] x k product (or one with smaller m and k) is not short of k splits, and the most that an
+// engine sets aside for it: two partial tiles per SM.
+size_t GemmF32ScratchBytes(size_t m, size_t n, size_t k);
+size_t GemmF32ScratchCap();
 
 }  // namespace cavs_b200
 #endif

@@ -157,6 +157,13 @@ Choice Choose(const GemmF32Args& g) {
   return c;
 }
 
+// The most k splits that Choose considers.
+size_t MaxSplits(size_t k) {
+  size_t z = 1;
+  while (z < 32 && 2 * z <= (k + 63) / 64) z *= 2;
+  return k >= 256 ? std::max(z, std::min<size_t>(16, k / 64)) : z;
+}
+
 int Check(const GemmF32Args& g) {
   CAVS_REQUIRE(g.m >= 0 && g.n >= 0 && g.k >= 0, CAVS_ERR_BAD_ARG, "gemm_f32: negative dimension");
   CAVS_REQUIRE(g.m == 0 || g.n == 0 || (g.a && g.b && g.c), CAVS_ERR_BAD_ARG, "gemm_f32: null pointer");
@@ -187,6 +194,9 @@ int Run(const GemmF32Args& g_in, int tile_n, int splits, cudaStream_t stream) {
 }
 
 }  // namespace
+
+size_t GemmF32ScratchBytes(size_t m, size_t n, size_t k) { return MaxSplits(k) > 1 ? MaxSplits(k) * m * n * sizeof(float) : 0; }
+size_t GemmF32ScratchCap() { return static_cast<size_t>(2) * SmCount() * 128 * 128 * sizeof(float); }
 
 double GemmF32Us(int m, int n, int k, size_t scratch_bytes) {
   GemmF32Args g;
