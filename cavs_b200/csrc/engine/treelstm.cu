@@ -431,8 +431,9 @@ double PerLevelUsF32(const cavs_treelstm* e, int rows, bool backward) {
 //         H = 32, two slots    7.8 / 10.8 at 2048, 2.5 / 2.9 at 4096, -9.0 / -9.9 at 8192
 //   bf16  H = 1024, two slots  5.7 / 12.1 at 16, 1.4 / 4.9 at 32, -6.5 / -7.4 at 64
 //         H = 512, one slot    5.3 / 4.7 at 64, 2.0 / 4.8 at 128, -4.0 / -4.0 at 256
-// fp32: by estimates of both; the margins keep out levels that the estimates' errors would make slower (over 300 sizes they
-// give away 100 of 5280 us; one product of rows and widths for all sizes gave away 290, up to 29 us in one level).
+// fp32: up to 128 rows below a number of multiply-adds (where no level of 300 sizes lost more than 1.5 us), else by estimates
+// of both sides, with margins that keep out levels that their errors would make slower.  The number of multiply-adds
+// alone, at any number of rows, lost up to 29 us in a level of 2048 rows at H = 75.
 // bf16: per level 11 us forward and 21 backward at H = 1024 (10 and 17 at 512), more without the fused loss head's streaming
 // cell; the plan's estimate and the line it is held against are both about 1.4 times that, and the line lies where the signs
 // above change (over 200 sizes it gives away 23 of the 2068 us that could be saved).
@@ -442,6 +443,7 @@ std::vector<NarrowRange> NarrowLevels(const cavs_treelstm* e, const cavs_treelst
   if (!e->narrow) return out;
   const int H = e->cfg.hidden, K = e->cfg.n_slots, n = bt.n_levels;
   const double bf16_line = 0.8 * (backward ? 16.0 + H / 75.0 : 13.0 + H / 200.0), f32_margin = backward ? 0.85 : 0.9;
+  const double f32_rows = std::min(128.0, (backward ? 6e7 : 1.2e8) / (static_cast<double>(H) * H * (3 + K)));
   auto rows = [&](int l) { return bt.level_off[l + 1] - bt.level_off[l]; };
   auto plan = [&](int r) { return e->bf16 ? PlanNarrowBf16(H, K, r, backward) : PlanNarrowF32(H, K, r, backward); };
   NarrowPlan wide;
@@ -453,7 +455,8 @@ std::vector<NarrowRange> NarrowLevels(const cavs_treelstm* e, const cavs_treelst
     wide = plan(seen);
     if (wide.w == 0) return out;   // slices and rows do not fit: fp32 H above 576 (two slots) to 768 (one) forward, 704 to 1024
                                    // backward; bf16 1184, forward 1152, 896 and 768 with two, three and four slots
-    if (e->bf16 ? wide.level_us <= bf16_line : NarrowLevelUsF32(wide, H, K, seen, backward) < f32_margin * PerLevelUsF32(e, seen, backward)) break;
+    if (e->bf16 ? wide.level_us <= bf16_line
+                : seen <= f32_rows || NarrowLevelUsF32(wide, H, K, seen, backward) < f32_margin * PerLevelUsF32(e, seen, backward)) break;
   }
   if (begin >= n || (e->bf16 && begin == n - 1)) return out;   // (a single bf16 level saves less than its launch costs)
   // Two launches where the upper levels are much narrower.  fp32: few rows want few hidden units per CTA, so that all CTAs
@@ -469,7 +472,7 @@ std::vector<NarrowRange> NarrowLevels(const cavs_treelstm* e, const cavs_treelst
       out.push_back({split, n, low});
     }
   }
-  if (!e->bf16 && n - begin <= 2) {   // the launches have to pay (three levels do: the narrower, the more a level saves)
+  if (!e->bf16 && n - begin <= 2 && rows(begin) > f32_rows) {   // one or two wide levels have to pay for their launches
     double gain = -9.0 * out.size();
     for (const NarrowRange& r : out)
       for (int l = r.begin; l < r.end && gain <= 0.0; ++l) gain += PerLevelUsF32(e, rows(l), backward) - NarrowLevelUsF32(r.plan, H, K, rows(l), backward);
