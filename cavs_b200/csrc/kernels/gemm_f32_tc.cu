@@ -233,12 +233,12 @@ __device__ __forceinline__ void DrainAdd(float (&acc)[kCols], uint32_t taddr) {
 }
 
 // One row of a tile's columns [col0, col0 + cols) in fp32, by one thread that waits for nobody: after an expired wait.
-__device__ __noinline__ void PlainRow(const GemmF32Args& g, float* c, long long ldc, int accumulate, int row, int col0, int cols, int k0,
+__device__ __noinline__ void PlainRow(const float* a, long long a_rs, long long a_cs, const float* b, long long b_rs, long long b_cs, int m, int n, float* c, long long ldc, int accumulate, int row, int col0, int cols, int k0,
                                       int k1) {
-  if (row >= g.m) return;
-  for (int j = col0; j < min(col0 + cols, g.n); ++j) {
+  if (row >= m) return;
+  for (int j = col0; j < min(col0 + cols, n); ++j) {
     float acc = 0.0f;
-    for (int k = k0; k < k1; ++k) acc = fmaf(g.a[row * g.a_rs + k * g.a_cs], g.b[k * g.b_rs + j * g.b_cs], acc);
+    for (int k = k0; k < k1; ++k) acc = fmaf(a[row * a_rs + k * a_cs], b[k * b_rs + j * b_cs], acc);
     float* dst = c + row * ldc + j;
     *dst = accumulate ? *dst + acc : acc;
   }
@@ -313,11 +313,10 @@ template <int kBN>
 __device__ __noinline__ void PlainTiles(const SplitParams& p) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
-  const uint32_t* words = reinterpret_cast<const uint32_t*>(smem + SplitSmem<kBN>::kBarOff) + 23;   // any mark, marks
-  if (words[0] == 0) return;
+  const uint32_t* marks = reinterpret_cast<const uint32_t*>(smem + SplitSmem<kBN>::kBarOff) + 24;
   const int tiles_n = (p.g.n + kBN - 1) / kBN, n_work = ((p.g.m + kBM - 1) / kBM) * tiles_n * p.n_splits;
   for (int i = 0; i < kMarks / 32; ++i)
-    for (uint32_t word = words[1 + i]; word != 0; word &= word - 1) {
+    for (uint32_t word = marks[i]; word != 0; word &= word - 1) {
       BlockPos b;
       b.w = blockIdx.x + (i * 32 + __ffs(word) - 1) * gridDim.x;
       if (i * 32 + __ffs(word) == kMarks || !SeekItem<kBN>(p, n_work, tiles_n, b)) continue;
@@ -327,8 +326,9 @@ __device__ __noinline__ void PlainTiles(const SplitParams& p) {
     }
 }
 
+// (A parameter whose address is taken is copied to the stack at entry unless it is a grid constant: 1 us of a product of 12.)
 template <int kBN, int kModeA, int kModeB>
-__global__ void __launch_bounds__(kF32Threads, 1) GemmF32SplitKernel(const SplitParams p) {
+__global__ void __launch_bounds__(kF32Threads, 1) GemmF32SplitKernel(const __grid_constant__ SplitParams p) {
   using S = SplitSmem<kBN>;
   constexpr int kCols = kBN / 2;   // columns per drain warp
   ChainRelease(p.chain_early);
@@ -487,7 +487,7 @@ __global__ void __launch_bounds__(kF32Threads, 1) GemmF32SplitKernel(const Split
       const int mark = min(b.t_local, kMarks - 1);
       const bool marked = *reinterpret_cast<volatile uint32_t*>(marks + (mark >> 5)) >> (mark & 31) & 1;
       if (!ok || marked) {   // marked: computed after all others, but for the tiles that share the last bit
-        if (!marked || mark == kMarks - 1) PlainRow(g, c, ldc, accumulate, row0 + lane, col_base, kCols, b.k0, min(g.k, b.k0 + b.kb_count * kBK));
+        if (!marked || mark == kMarks - 1) PlainRow(g.a, g.a_rs, g.a_cs, g.b, g.b_rs, g.b_cs, g.m, g.n, c, ldc, accumulate, row0 + lane, col_base, kCols, b.k0, min(g.k, b.k0 + b.kb_count * kBK));
         continue;
       }
       const bool vec = (ldc & 3) == 0 && (reinterpret_cast<uintptr_t>(c) & 15) == 0;
@@ -540,7 +540,10 @@ __global__ void __launch_bounds__(kF32Threads, 1) GemmF32SplitKernel(const Split
   __syncthreads();
   if (warp == 0)
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(4 * kBN));
-  PlainTiles<kBN>(p);
+  // (asked before the call, which would save registers first; the address is formed anew, not kept)
+  uint32_t any;
+  asm volatile("ld.shared.b32 %0, [%1];" : "=r"(any) : "r"(((SmemAddr(smem_raw) + 1023) & ~1023u) + S::kBarOff + 23 * 4) : "memory");
+  if (any != 0) PlainTiles<kBN>(p);
 }
 
 ReadMode ReadModeOf(const float* base, int rows, long long row_stride, int k, long long k_stride, int tile_rows) {
