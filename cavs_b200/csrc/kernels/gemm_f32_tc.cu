@@ -17,11 +17,12 @@
 // where all values lie within 1 % of 2 at k = 14474 (1.7e-6 -> 1.8e-6), and where results lie below 2^-120, whose corrections
 // reach fp32's subnormals (2^-124: 4.0e-7 -> 4.6e-7).
 //
-// What bounds it: 132 TFLOP/s of fp32 products at [14474, 512] x [512, 10000] (5800 us with the FFMA kernel, 1124 with
-// this one), 111 with k = 10000, 99 with k = 14474 and both operands strided along k.  Six MMAs per product stand
+// What bounds it: 127 TFLOP/s of fp32 products at [14474, 512] x [512, 10000] (5846 us with the FFMA kernel, 1163 with
+// this one), 110 with k = 10000 (6858, 1352), 93 with k = 14474 and both operands strided along k (6989, 1598).  Of these
+// 0, 1 and 9 % are the price of looking at every split for bits that its three parts do not hold.  Six MMAs per product stand
 // against operands that must be split by ordinary instructions.  Per 128 x 128 x 64
 // block the MMAs take 1536 clocks of the tensor pipe, the split of 2 x 8192 values ~1000 issue slots of each scheduler; the block takes 4200,
-// because the splitting warps wait for their loads (long-scoreboard stalls, tensor pipe 34 % busy).  Tried against that:
+// because the splitting warps wait for their loads (long-scoreboard stalls, tensor pipe 35 % busy).  Tried against that:
 // reloading run by run, a second set of registers under setmaxnreg, clamped instead of predicated addresses -- all slower.
 // So the split is done in the kernel (no extra pass over memory, no copies of the weights to keep) by eight warps that
 // load the next block's values while they convert this one's, beside eight warps that issue the MMAs and drain the
@@ -326,7 +327,8 @@ __device__ __noinline__ void PlainTiles(const SplitParams& p) {
     }
 }
 
-// (A parameter whose address is taken is copied to the stack at entry unless it is a grid constant: 1 us of a product of 12.)
+// (A parameter whose address is taken is copied to the stack at entry unless it is a grid constant: with the marks asked before
+// PlainTiles is called, [256, 512] x [512, 1536] went from 20.4 to 18.5 us, [595, 150] x [150, 450] from 18.4 to 16.4.)
 template <int kBN, int kModeA, int kModeB>
 __global__ void __launch_bounds__(kF32Threads, 1) GemmF32SplitKernel(const __grid_constant__ SplitParams p) {
   using S = SplitSmem<kBN>;

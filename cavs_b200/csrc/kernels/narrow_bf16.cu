@@ -1,7 +1,7 @@
 // The narrow levels of the bf16 Tree-LSTM in one launch per direction (see narrow_f32.cu for the scheme): a persistent
 // grid walks the levels with a bounded grid barrier between them, each CTA keeps its eight hidden units' slice of the
 // recurrent weights in shared memory.  One child slot, H = 512, 49 rows on average: 15.6 -> 6.1 us per level forward,
-// 23.6 -> 9 us backward; two stacked layers of 60 levels 3.78 -> 2.41 ms per step.
+// 23.6 -> 9 us backward; two stacked layers of 60 levels 3.80 -> 2.50 ms per step.
 //
 // Level by level a narrow level costs 16 us forward (child gather, both gate products in one launch, cell) and 23 us
 // backward (cell gradient, two products) at H = 512, of which the tensor cores work a fraction of a microsecond.

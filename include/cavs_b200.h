@@ -315,7 +315,8 @@ CAVS_API int cavs_allgather(const void* send, void* recv, size_t bytes_per_rank,
 typedef struct cavs_treelstm cavs_treelstm;
 typedef struct cavs_treelstm_config {
   int hidden, embed, vocab, classes, n_slots;
-  int gemm_bf16;       /* 1: gate GEMMs on tcgen05 with bf16 operands; 0: fp32 GEMMs on the CUDA cores */
+  int gemm_bf16;       /* 1: gate GEMMs on tcgen05 with bf16 operands; 0: fp32 operands (small products on the CUDA cores,
+                          larger ones on tcgen05, each value split into three bf16 parts) */
   int max_vertices;    /* capacity: vertices per batch */
   int max_level_rows;  /* capacity: rows of the widest level */
 } cavs_treelstm_config;

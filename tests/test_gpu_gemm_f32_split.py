@@ -57,7 +57,7 @@ def test_accumulate(cuda, n):
 
 
 def test_values_without_a_finite_split(cuda):
-    # infinities, NaN and values that round to infinity in bf16 give what fp32 arithmetic gives; tiny ones are not lost
+    # infinities, NaN and values that round to infinity in bf16 give what fp32 arithmetic gives (tiny ones: test_gpu_gemm_f32_tiled.py)
     g = torch.Generator().manual_seed(5)
     A, B = torch.randn((600, 512), generator=g), torch.randn((512, 640), generator=g)
     B[7] *= 0.01          # (3.4e38 times it stays in range)
